@@ -2,6 +2,7 @@
 // translation units of libd4core.so.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -15,12 +16,12 @@ namespace d4 {
 constexpr int kTile = 32;          // pair tile edge
 constexpr int kLuNb = 32;          // LU block width (FP64 path)
 // Cooperative LU buffers: per launch one mask word per possible pass, then
-// the FP64 form's schedule words (tickets, strip counters, look-ahead epoch);
-// after the two Q halves (2 x n x 32) the published diagonal block and its
-// reciprocals.
+// the FP64 form's schedule words (strip counters, look-ahead epoch); after the
+// two Q halves (2 x n x 32) the FP64 form's two U12 halves (2 x 32 x n) and the
+// published diagonal block with its reciprocals.
 constexpr int lu_pass_words(int nblk) { return nblk * 33 + 8; }
 constexpr int lu_mask_words_for(int nblk) { return lu_pass_words(nblk) + nblk + 64; }
-constexpr int kLuDiagWords = kLuNb * (kLuNb + 1) + kLuNb + kLuNb * kLuNb;
+constexpr int kLuDiagWords = kLuNb * (kLuNb + 1) + kLuNb;
 constexpr int kSolveThreads = 1024;
 constexpr int kMaxSolveN = 8192;   // x and g of the one-CTA solve live in shared memory
 
@@ -38,8 +39,14 @@ enum FlagSlot {
 // wait gave up.
 constexpr int kWaveErrRows = 5;
 
+// Tensor maps of the FP64 LU's matrix and U12 buffer (d4_lu_coop64.cu).
+struct LuMaps {
+    CUtensorMap a, u;
+};
+
 // Buffers of one LU factorisation (factors, pivot bookkeeping, flags).
 struct LuBufs {
+    const LuMaps *maps = nullptr;  // of LU and Q's U12 halves
     double *LU = nullptr, *P0 = nullptr, *Q = nullptr;
     unsigned *mask = nullptr, *bar = nullptr;
     int *flags = nullptr, *perm = nullptr, *piv = nullptr;
@@ -156,6 +163,7 @@ struct Ctx {
     double *lu_p0 = nullptr, *lu_q = nullptr;
     unsigned *lu_mask = nullptr, *lu_bar = nullptr;
     int lu_mask_words = 0, lu_grid = 0;
+    LuMaps lu_maps, lub_maps;  // of LU and of stage I's lub.LU
 
     // mixed form: FP32 matrix and factors, FP64 accumulators and refinement
     float *A32 = nullptr, *LU32 = nullptr, *lu32_p0 = nullptr, *lu32_q = nullptr;
@@ -289,6 +297,7 @@ int factor64(Ctx &c);                 // d4_lu_coop64.cu
 void factor64_async(Ctx &c, const LuBufs &L, const double *A, int grid, cudaStream_t st,
                     cudaEvent_t after_copy);
 LuBufs primary_lu(Ctx &c);
+void lu_encode_maps(LuMaps &m, double *A, double *U, int n);
 // Adds one factorisation's pass and swap counts (its flag words) to the
 // context's counters.
 inline void count_lu(Ctx &c, const int *fl) {

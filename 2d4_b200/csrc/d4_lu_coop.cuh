@@ -1,5 +1,10 @@
-// d4_lu_coop.cuh: the cooperative LU kernel, templated on the scalar type
-// (double: plain form, --fmad=false; float: mixed form).  See d4_lu_coop64.cu.
+// d4_lu_coop.cuh: the mixed form's cooperative FP32 LU with exact partial
+// pivoting.  Per block of 32 columns a pass eliminates without pivoting, from a
+// saved copy P0 with the swaps found so far, and flags the columns where partial
+// pivoting would have swapped; a flagged pass finds the first one's exact pivot
+// and repeats (the FP64 form's scheme, d4_lu_exact.cuh).  Then the swaps and
+// U12 = L11^-1 A12 on the other columns, and the trailing update on the tensor
+// cores.
 #pragma once
 #include <cstdint>
 #include <type_traits>
@@ -16,8 +21,7 @@ constexpr long long kSpinLimit = 1ll << 24;  // x >= 64 ns each: > 1 s
 constexpr int kGenWord = 32;
 // Dynamic shared memory: the narrow last block's rows (a row of NB + 1 entries
 // per thread) and the diagonal block's pre-division values (NB rows) during a
-// pass, the trailing update's second piece buffer during the update; for the
-// FP32 form after them the four
+// pass; after them the four
 // tensor-core operand tiles (L21 and U12 as TF32 hi and lo parts, 16 KiB each,
 // 1 KiB aligned) plus the MMA completion barrier and the TMEM address slot.
 constexpr size_t kOpTileBytes = 128 * NB * 4;
@@ -42,19 +46,7 @@ struct CoopArgs {
     int *piv;        // n pivot rows
     int *flags;      // kFlagSingular, kFlagBarrierTimeout, kFlagPasses, kFlagSwaps
     unsigned *bar;   // grid barrier: [0] arrivals, [kGenWord] generation
-    // FP64 form only (look-ahead of the next diagonal block during the
-    // trailing update), zeroed before the launch: per block kb the update's
-    // finished strip-0 tiles [kb]; [nblk] the last block whose diagonal block
-    // is published
-    unsigned *sched;
-    T *dg;           // kLuDiagWords: see kDiagWords (null in the FP32 form)
 };
-
-// dg: the published diagonal block s (NB x (NB + 1)), its reciprocals rs (NB),
-// then the next diagonal block's entries before the update (NB x NB, by column)
-constexpr int kDiagWords = NB * (NB + 1) + NB;
-constexpr int kSnapOffset = kDiagWords;
-static_assert(kDiagWords + NB * NB == kLuDiagWords && NB == kLuNb, "buffer sizes in d4_internal.h");
 
 __device__ __forceinline__ unsigned ld_acq(const unsigned *p) {
     unsigned v;
@@ -95,27 +87,6 @@ static __device__ void grid_barrier(unsigned *bar, int *flags, unsigned &gen, in
     __syncthreads();
 }
 
-__device__ __forceinline__ void st_rel(unsigned *p, unsigned v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// Thread 0: wait until *p >= target, bounded as the grid barrier is (a CTA
-// that gives up records kFlagBarrierTimeout and stops waiting for good).
-__device__ __forceinline__ void wait_ge(const unsigned *p, unsigned target, int *flags,
-                                        int *dead_s) {
-    if (*dead_s) return;
-    long long spins = 0;
-    while (ld_acq(p) < target) {
-        __nanosleep(32);
-        if ((++spins & 255) == 0 &&
-            (spins > kSpinLimit || ld_acq((const unsigned *)&flags[kFlagBarrierTimeout]))) {
-            atomicOr(&flags[kFlagBarrierTimeout], 1);
-            *dead_s = 1;
-            return;
-        }
-    }
-}
-
 // Source row in P0 of position r after the block's transpositions (applied in
 // order to the arrangement): walk the list backwards.
 __device__ __forceinline__ int src_row(int r, const int *sa, const int *sb, int ns) {
@@ -138,17 +109,16 @@ template <typename T>
 __device__ __noinline__ unsigned diag_block(const CoopArgs<T> &a, T *Q, T (*s)[NB + 1],
                                             T *rs, T (*qbuf)[NB + 1], int k0, int kw,
                                             const int *sa, const int *sb, int ns, unsigned skip,
-                                            bool write_q, bool preloaded = false) {
+                                            bool write_q) {
     const int n = a.n;
     const int tid = threadIdx.x;
     unsigned msk = 0;
-    if (!preloaded)
-        for (int t = tid; t < NB * NB; t += kThreads) {
-            const int r = t % NB, k = t / NB;
-            T v = 0.0;
-            if (r < kw && k < kw) v = a.P0[(size_t)src_row(k0 + r, sa, sb, ns) + (size_t)k * n];
-            s[r][k] = v;
-        }
+    for (int t = tid; t < NB * NB; t += kThreads) {
+        const int r = t % NB, k = t / NB;
+        T v = 0.0;
+        if (r < kw && k < kw) v = a.P0[(size_t)src_row(k0 + r, sa, sb, ns) + (size_t)k * n];
+        s[r][k] = v;
+    }
     __syncthreads();
     for (int k = 0; k < kw; ++k) {
         const T d = s[k][k];
@@ -298,8 +268,7 @@ __device__ __noinline__ unsigned rows_below(const CoopArgs<T> &a, T *Q,
 // The block's row swaps on every other column, then U12 = L11^-1 A12 on the
 // columns right of the block, a warp per column: lane r holds row r, column
 // k's value reaches the lanes below by shuffle (u_kj == 0 skips its updates,
-// as the oracle does).  The FP64 form also keeps the next diagonal block's
-// entries (after the swaps, before the update) for the look-ahead.
+// as the oracle does).
 template <typename T>
 __device__ __noinline__ void finish_cols(const CoopArgs<T> &a, const T (*s)[NB + 1], int k0,
                                          int kw, const int *sa, const int *sb, int ns) {
@@ -318,10 +287,6 @@ __device__ __noinline__ void finish_cols(const CoopArgs<T> &a, const T (*s)[NB +
                 }
             }
             __syncwarp();
-            if (a.dg && j >= k0 + kw && j < k0 + kw + NB) {
-                const int nk0 = k0 + kw;
-                if (nk0 + lane < n) a.dg[kSnapOffset + (j - nk0) * NB + lane] = cj[nk0 + lane];
-            }
             if (j >= k0 + kw) {
                 T v = lane < kw ? cj[k0 + lane] : 0.0;
                 for (int k = 0; k < kw; ++k) {
@@ -330,159 +295,6 @@ __device__ __noinline__ void finish_cols(const CoopArgs<T> &a, const T (*s)[NB +
                 }
                 if (lane < kw) cj[k0 + lane] = v;
             }
-        }
-    }
-}
-
-__device__ __forceinline__ void cp_async8(void *smem, const void *gmem, bool valid) {
-    // 8 bytes global -> shared without registers; zero-filled when !valid
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(
-                     (unsigned)__cvta_generic_to_shared(smem)),
-                 "l"(gmem), "r"(valid ? 8 : 0)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-
-// Trailing update A22 -= L21 U12 of the plain form, every entry in the
-// oracle's order (k ascending, product and difference rounded separately);
-// tiles holding the next block's columns (strip 0) also refresh P0.  64 x 64
-// tiles, 4 x 4 entries per thread.  While a tile computes, the next tile's L21
-// and U12 pieces stream into the other shared-memory buffer (cp.async) and its
-// entries into registers.
-//
-// Look-ahead: the last CTA takes no tile (unless it is the only one).  It
-// forms the next block's diagonal block itself from A, L21 and U12 (the same
-// operations in the same order as the tile that owns it, so the same values),
-// eliminates it as diag_block does for the next block's first pass (no swaps
-// yet) and publishes it: s and rs to dg, pre-division values to Q, flags into
-// the next pass's mask word.  The next pass starts without a grid barrier,
-// once the diagonal block is published and the strip-0 tiles (P0) are done.
-template <typename T>
-__device__ __noinline__ void update_la(const CoopArgs<T> &a, int k0, int kw, int kb, int pass,
-                                       T *buf0, T *buf1, T (*s)[NB + 1], T *rs,
-                                       T (*qbuf)[NB + 1], const int *sa, const int *sb,
-                                       unsigned *la_mask_s) {
-    constexpr int kLd = 64 + 1;          // row stride of the L and U pieces
-    constexpr int kPiece = NB * kLd;     // one piece (L or U)
-    const int n = a.n, tid = threadIdx.x, cta = blockIdx.x, G = gridDim.x;
-    const int nblk = (n + NB - 1) / NB;
-    const int base = k0 + kw, rest = n - base;
-    const int tb = (rest + 63) / 64;
-    const int nk0 = base, nkw = min(NB, n - base);  // next block's columns
-    const int tr = tid % 16, tc = tid / 16;
-    const int ntiles = tb * tb;
-    const int gt = G > 1 ? G - 1 : 1;  // CTAs that take tiles
-    if (cta == G - 1) {
-        // the next block's diagonal block: L and U pieces, then 4 entries per thread
-        T *Lp = buf0, *Up = buf0 + NB * (NB + 1);
-        for (int t = tid; t < NB * NB; t += kThreads) {
-            const int r = t % NB, k = t / NB;
-            Lp[k * (NB + 1) + r] = (r < nkw && k < kw) ? a.A[(size_t)(nk0 + r) + (size_t)(k0 + k) * n] : T(0);
-            const int k2 = t % NB, c = t / NB;
-            Up[k2 * (NB + 1) + c] = (c < nkw && k2 < kw) ? a.A[(size_t)(k0 + k2) + (size_t)(nk0 + c) * n] : T(0);
-        }
-        // the entries before the update come from the snapshot finish_cols
-        // took: the tile that owns them may already have overwritten A
-        T v[NB * NB / kThreads];
-#pragma unroll
-        for (int e = 0; e < NB * NB / kThreads; ++e) {
-            const int t = tid + e * kThreads, r = t % NB, c = t / NB;
-            v[e] = (r < nkw && c < nkw) ? __ldcg(a.dg + kSnapOffset + c * NB + r) : T(0);
-        }
-        __syncthreads();
-        for (int k = 0; k < kw; ++k) {
-#pragma unroll
-            for (int e = 0; e < NB * NB / kThreads; ++e) {
-                const int t = tid + e * kThreads, r = t % NB, c = t / NB;
-                v[e] = v[e] - Lp[k * (NB + 1) + r] * Up[k * (NB + 1) + c];
-            }
-        }
-#pragma unroll
-        for (int e = 0; e < NB * NB / kThreads; ++e) {
-            const int t = tid + e * kThreads;
-            s[t % NB][t / NB] = v[e];
-        }
-        if (tid == 0) *la_mask_s = 0;
-        T *Qn = a.Q + (size_t)(pass & 1) * n * NB;
-        const unsigned m = diag_block(a, Qn, s, rs, qbuf, nk0, nkw, sa, sb, 0, 0u, true, true);
-        if (m) atomicOr(la_mask_s, m);
-        for (int t = tid; t < kDiagWords; t += kThreads)
-            a.dg[t] = t < NB * (NB + 1) ? s[t / (NB + 1)][t % (NB + 1)] : rs[t - NB * (NB + 1)];
-        __syncthreads();
-        if (tid == 0) {
-            if (*la_mask_s) atomicOr(&a.mask[pass], *la_mask_s);
-            __threadfence();
-            st_rel(a.sched + nblk, (unsigned)(kb + 1));
-        }
-        if (G > 1) return;
-    }
-    T pa[4][4];
-    auto stage = [&](int tile, T *buf) {
-        const int i0 = base + (tile % tb) * 64, j0 = base + (tile / tb) * 64;
-        T *Ls = buf, *Us = buf + kPiece;
-#pragma unroll
-        for (int r = 0; r < 64 * NB / kThreads; ++r) {
-            const int t = tid + r * kThreads;
-            const int ii = t % 64, k = t / 64;
-            const bool vl = k < kw && i0 + ii < n;
-            cp_async8(Ls + k * kLd + ii, vl ? a.A + (size_t)(i0 + ii) + (size_t)(k0 + k) * n : a.A, vl);
-            const int k2 = t % NB, jj = t / NB;
-            const bool vu = k2 < kw && j0 + jj < n;
-            cp_async8(Us + k2 * kLd + jj, vu ? a.A + (size_t)(k0 + k2) + (size_t)(j0 + jj) * n : a.A, vu);
-        }
-        cp_async_commit();
-#pragma unroll
-        for (int p = 0; p < 4; ++p)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int gi = i0 + tr + 16 * p, gj = j0 + tc + 16 * q;
-                pa[p][q] = (gi < n && gj < n) ? a.A[(size_t)gi + (size_t)gj * n] : T(0);
-            }
-    };
-    if (cta < ntiles) stage(cta, buf0);
-    int par = 0;
-    for (int tile = cta; tile < ntiles; tile += gt, par ^= 1) {
-        const int i0 = base + (tile % tb) * 64, j0 = base + (tile / tb) * 64;
-        const T *Ls = par ? buf1 : buf0;
-        const T *Us = Ls + kPiece;
-        T acc[4][4];
-#pragma unroll
-        for (int p = 0; p < 4; ++p)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) acc[p][q] = pa[p][q];
-        cp_async_wait_all();
-        __syncthreads();  // this tile's pieces are in; the other buffer is free
-        if (tile + gt < ntiles) stage(tile + gt, par ? buf0 : buf1);
-#pragma unroll 2
-        for (int k = 0; k < kw; ++k) {
-            T lv[4], uv[4];
-#pragma unroll
-            for (int p = 0; p < 4; ++p) lv[p] = Ls[k * kLd + tr + 16 * p];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) uv[q] = Us[k * kLd + tc + 16 * q];
-#pragma unroll
-            for (int p = 0; p < 4; ++p)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) acc[p][q] = acc[p][q] - lv[p] * uv[q];
-        }
-#pragma unroll
-        for (int p = 0; p < 4; ++p)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int gi = i0 + tr + 16 * p, gj = j0 + tc + 16 * q;
-                if (gi < n && gj < n) {
-                    a.A[(size_t)gi + (size_t)gj * n] = acc[p][q];
-                    if (gj >= nk0 && gj < nk0 + nkw)
-                        a.P0[(size_t)gi + (size_t)(gj - nk0) * n] = acc[p][q];
-                }
-            }
-        // products done with this buffer before it is refilled; a strip-0
-        // tile's stores are in before it is counted
-        __syncthreads();
-        if (tile < tb && tid == 0) {
-            __threadfence();
-            atomicAdd(a.sched + kb, 1u);
         }
     }
 }
@@ -585,7 +397,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_lu_coop(CoopArgs<T> a) {
     T *rowbuf = reinterpret_cast<T *>(rowbuf_raw);  // see kRowBufRaw
     __shared__ T s[NB][NB + 1];           // diagonal block (rows = positions k0..k0+31)
     __shared__ T rs[NB];                  // RN(1 / pivot) of the block's columns
-    __shared__ __align__(16) T LUs[2 * NB * (64 + 1)];  // update: L21 and U12 pieces (buffer 0)
     __shared__ int sa[NB], sb[NB];        // swap list of the block (positions)
     __shared__ unsigned skip_mask;        // singular columns (skipped)
     __shared__ int ns_s;
@@ -593,7 +404,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_lu_coop(CoopArgs<T> a) {
     __shared__ T red_v[kThreads / 32];
     __shared__ int red_i[kThreads / 32];
     __shared__ int dead_s;
-    __shared__ unsigned la_mask_s;        // look-ahead: flags of the diagonal block
 
     const int n = a.n;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -602,12 +412,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_lu_coop(CoopArgs<T> a) {
     if (tid == 0) dead_s = 0;
     const int nblk = (n + NB - 1) / NB;
     for (int i = cta * kThreads + tid; i < n; i += G * kThreads) a.perm[i] = i;
-    constexpr bool kTc = std::is_same<T, float>::value;
+    static_assert(std::is_same<T, float>::value, "the FP64 form is d4_lu_exact.cuh");
     unsigned char *tc_base = rowbuf_raw + kTcOffset<T>();
     uint64_t *tc_mbar = reinterpret_cast<uint64_t *>(tc_base + 4 * kOpTileBytes);
     uint32_t *tc_slot = reinterpret_cast<uint32_t *>(tc_base + 4 * kOpTileBytes + 64);
     uint32_t tmem = 0, tc_phase = 0;
-    if (kTc) {
+    {
         if (warp == 0) {
             asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 128;"
                          ::"r"(tc::smem_u32(tc_slot)) : "memory");
@@ -641,7 +451,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_lu_coop(CoopArgs<T> a) {
         }
         __syncthreads();
         int scan_from = 0;
-        bool first = true;
         // ------------------------------------------------------------ passes
         for (;;) {
             const int par = pass & 1;
@@ -650,29 +459,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_lu_coop(CoopArgs<T> a) {
             const unsigned skip = skip_mask;
             if (tid == 0) cta_mask = 0;
             unsigned my_mask = 0;
-            if (!kTc && kb > 0 && first) {
-                // the diagonal block published by the previous update's
-                // look-ahead, once that update's strip 0 (P0) is done too
-                if (tid == 0) {
-                    wait_ge(a.sched + nblk, (unsigned)kb, a.flags, &dead_s);
-                    wait_ge(a.sched + (kb - 1), (unsigned)((n - k0 + 63) / 64), a.flags, &dead_s);
-                }
-                __syncthreads();
-                for (int t = tid; t < kDiagWords; t += kThreads) {
-                    const T v = __ldcg(a.dg + t);
-                    if (t < NB * (NB + 1))
-                        s[t / (NB + 1)][t % (NB + 1)] = v;
-                    else
-                        rs[t - NB * (NB + 1)] = v;
-                }
-                __syncthreads();
-            } else {
-                // diagonal block, redundantly in every CTA
-                my_mask = diag_block(a, Q, s, rs,
-                                     reinterpret_cast<T (*)[NB + 1]>(rowbuf + kThreads * (NB + 1)),
-                                     k0, kw, sa, sb, ns, skip, cta == 0);
-            }
-            first = false;
+            // diagonal block, redundantly in every CTA
+            my_mask = diag_block(a, Q, s, rs,
+                                 reinterpret_cast<T (*)[NB + 1]>(rowbuf + kThreads * (NB + 1)), k0,
+                                 kw, sa, sb, ns, skip, cta == 0);
             my_mask |= rows_below(a, Q, s, rs, rowbuf, k0, kw, sa, sb, ns, skip);
             if (my_mask) atomicOr(&cta_mask, my_mask);
             __syncthreads();
@@ -759,7 +549,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_lu_coop(CoopArgs<T> a) {
         // ---------------------------------------------------------- update
         const int base = k0 + kw;
         const int rest = n - base;
-        if (kTc && rest > 0) {
+        if (rest > 0) {
             const int nk0 = base, nkw = min(NB, n - base);  // next block's columns
             const int tb = (rest + 127) / 128;
             float *Ahi = reinterpret_cast<float *>(tc_base);
@@ -849,23 +639,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_lu_coop(CoopArgs<T> a) {
                 tc::fence_before();
                 __syncthreads();
             }
-        } else if (rest > 0) {
-            // buffer 1 reuses the panel's buffers; rows of the next block's
-            // columns above the trailing matrix are never read from P0
-            // (positions >= nk0 only)
-            update_la(a, k0, kw, kb, pass, LUs, rowbuf, s, rs,
-                      reinterpret_cast<T (*)[NB + 1]>(rowbuf + kThreads * (NB + 1)), sa, sb,
-                      &la_mask_s);
         }
-        // FP64 form: the next pass waits for the look-ahead and strip 0 only;
-        // the pass barrier then also closes this update
-        if (kTc) grid_barrier(a.bar, a.flags, gen, &dead_s);
+        grid_barrier(a.bar, a.flags, gen, &dead_s);
     }
     if (cta == 0 && tid == 0) {
         a.flags[kFlagPasses] = pass;
         a.flags[kFlagSwaps] = swaps;
     }
-    if (kTc) {
+    {
         tc::fence_before();
         __syncthreads();
         if (warp == 0)

@@ -1,67 +1,62 @@
-// d4_lu_coop64.cu: FP64 LU with partial pivoting as one persistent kernel
-// (compiled with --fmad=false).
-//
-// Same result, bit for bit, as the oracle's right-looking Gaussian elimination
-// with partial pivoting (first index of the largest |a_ik| wins; an exact zero
-// pivot skips its column and marks the matrix singular), which stands in for
-// umfpack_di_numeric (src/simulation.cpp:635-640).  Every entry keeps its
-// update sequence: a_ij -= l_ik * u_kj for k ascending, product and difference
-// rounded separately.
-//
-// Schedule.  The matrix is processed in 32-column blocks by all CTAs of a
-// cooperative launch:
-//   pass   every CTA eliminates the block's 32 columns for its rows below the
-//          diagonal block, WITHOUT pivoting, starting from a saved copy P0 of
-//          the block's columns with the swaps found so far applied.  The 32x32
-//          diagonal block of a block's first pass was eliminated and published
-//          by the previous update's look-ahead; for block 0 and for passes
-//          after a swap every CTA eliminates it redundantly in shared memory.
-//          Pre-division values go to Q; a 32-bit mask records the columns
-//          where partial pivoting would have swapped (some |a_ik| > |a_kk|) or
-//          met a zero pivot.  A grid barrier ends the pass.
-//   decide every CTA reads the mask.  Empty: the pass is exact, go on.
-//          Otherwise the first flagged column k* gets its exact pivot from Q
-//          (first max), the swap (or the singular skip) is appended to the
-//          block's list and the pass repeats.  A row swap at column k commutes
-//          with the updates of earlier columns, so applying the list to P0 up
-//          front is exact.
-//   finish CTAs write their rows' multipliers, apply the block's swaps to the
-//          other columns and solve U12 = L11^-1 A12 (warp per column), keeping
-//          the next diagonal block's entries (after the swaps) aside; grid
-//          barrier.
-//   update trailing A22 -= L21 U12 in 64x64 tiles on every CTA but the last,
-//          the next tile's operands loaded while the current one computes;
-//          tiles that hold the next block's columns also refresh P0 and are
-//          counted.  The last CTA forms the next diagonal block from the kept
-//          entries, L21 and U12 (the same operations in the same order as the
-//          tile that owns it), eliminates it and publishes it.  The oracle
-//          skips an update whose u_kj is exactly 0; here it is applied
-//          (x - l*0 == x for finite l, and the multipliers of an accepted pass
-//          are finite: |l| <= 1), so the factors agree bit for bit for every
-//          finite matrix.
-// The next block's first pass waits for the publication and the P0 tiles
-// only, so the update needs no grid barrier of its own and the diagonal block
-// leaves the critical path while the update runs.  A block without swaps
-// costs one pass and two grid barriers.  Every wait is bounded: after
-// kSpinLimit polls a CTA records an error and stops waiting, so a launch
-// always ends.
-#include "d4_lu_coop.cuh"
+// d4_lu_coop64.cu: host side of the FP64 LU with partial pivoting
+// (d4_lu_exact.cuh, compiled with --fmad=false).
+
+#include "d4_lu_exact.cuh"
 
 namespace d4 {
+
+namespace lux {
+
+__global__ void __launch_bounds__(kThreads, 1)
+    k_lu_grid(Args a, const __grid_constant__ LuMaps maps, unsigned long long *bar) {
+    a.map_a = &maps.a;
+    a.map_u = &maps.u;
+    factor(a, GridGroup{bar, 0u, 0u, false});
+}
+
+}  // namespace lux
+
+// Tensor maps of a factorisation's buffers: A (n x n, column-major) and the two
+// U12 halves (64 rows of n).
+void lu_encode_maps(LuMaps &m, double *A, double *U, int n) {
+    using Encode = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
+                                const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
+                                const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static const Encode encode = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) !=
+                cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            return (Encode) nullptr;
+        return reinterpret_cast<Encode>(p);
+    }();
+    if (!encode) throw StateError("cuTensorMapEncodeTiled not available");
+    auto one = [&](CUtensorMap &t, double *base, int rows, int box_x, int box_y) {
+        const cuuint64_t dims[2] = {(cuuint64_t)n, (cuuint64_t)rows};
+        const cuuint64_t strides[1] = {(cuuint64_t)n * sizeof(double)};
+        const cuuint32_t box[2] = {(cuuint32_t)box_x, (cuuint32_t)box_y}, step[2] = {1, 1};
+        if (encode(&t, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, base, dims, strides, box, step,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            throw StateError("cuTensorMapEncodeTiled failed");
+    };
+    one(m.a, A, n, lux::kBoxR, lux::kBoxC);
+    one(m.u, U, 2 * lux::NB, lux::kBoxC, lux::NB);
+}
 
 int coop_grid_size(int n) {
     int dev = 0, sms = 0, per_sm = 0;
     D4_CUDA_OK(cudaGetDevice(&dev));
     D4_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    D4_CUDA_OK(cudaFuncSetAttribute(coop::k_lu_coop<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)coop::kRowBufBytes<double>()));
-    D4_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, coop::k_lu_coop<double>, coop::kThreads,
-                                                             coop::kRowBufBytes<double>()));
-    int g = sms * (per_sm < 1 ? 1 : per_sm);
-    // enough threads for one row below the diagonal block per thread
-    const int need = (n + coop::kThreads - 1) / coop::kThreads;
-    if (g < need) return -1;
-    return g;
+    const int bytes = (int)sizeof(lux::Smem);
+    D4_CUDA_OK(cudaFuncSetAttribute(lux::k_lu_grid, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    bytes));
+    D4_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lux::k_lu_grid,
+                                                             lux::kThreads, bytes));
+    return per_sm < 1 ? -1 : sms * per_sm;
 }
 
 // Factorises A into L.LU on `st` with `grid` CTAs, without waiting: flags
@@ -76,23 +71,23 @@ void factor64_async(Ctx &c, const LuBufs &L, const double *A, int grid, cudaStre
     D4_CUDA_OK(cudaMemsetAsync(L.mask, 0, sizeof(unsigned) * c.lu_mask_words, st));
     D4_CUDA_OK(cudaMemcpyAsync(L.LU, A, bytes, cudaMemcpyDeviceToDevice, st));
     if (after_copy) D4_CUDA_OK(cudaEventRecord(after_copy, st));
-    coop::CoopArgs<double> a;
+    lux::Args a;
     a.n = n;
     a.A = L.LU;
     a.P0 = L.P0;
     a.Q = L.Q;
+    a.U = L.Q + (size_t)n * 64;
+    a.dg = L.Q + (size_t)n * 128;
     a.mask = L.mask;
+    a.sched = L.mask + lu_pass_words((n + kLuNb - 1) / kLuNb);
+    a.perm = L.perm;
     a.piv = L.piv;
     a.flags = L.flags;
-    a.bar = L.bar;
-    a.perm = L.perm;
-    a.sched = L.mask + lu_pass_words((n + kLuNb - 1) / kLuNb);
-    a.dg = L.Q + (size_t)n * 64;
-    void *args[] = {(void *)&a};
-    D4_CUDA_OK(cudaLaunchCooperativeKernel((const void *)coop::k_lu_coop<double>, dim3(grid),
-                                           dim3(coop::kThreads), args,
-                                           coop::kRowBufBytes<double>(), st));
-    check_launch("k_lu_coop<double>");
+    unsigned long long *bar = reinterpret_cast<unsigned long long *>(L.bar);
+    void *args[] = {(void *)&a, (void *)L.maps, (void *)&bar};
+    D4_CUDA_OK(cudaLaunchCooperativeKernel((const void *)lux::k_lu_grid, dim3(grid),
+                                           dim3(lux::kThreads), args, sizeof(lux::Smem), st));
+    check_launch("k_lu_grid");
 }
 
 LuBufs primary_lu(Ctx &c) {
@@ -105,6 +100,7 @@ LuBufs primary_lu(Ctx &c) {
     L.flags = c.flags;
     L.perm = c.perm;
     L.piv = c.piv;
+    L.maps = &c.lu_maps;
     return L;
 }
 

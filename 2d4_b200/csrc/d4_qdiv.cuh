@@ -35,18 +35,20 @@ __device__ __forceinline__ T recip(T b) {
     return in_range(b) ? T(1) / b : T(0);
 }
 
+// The division itself, out of line: taken outside the window only.
+static __device__ __noinline__ double slow_div(double a, double b) { return a / b; }
+
 // A zero numerator over an in-window divisor gives a y: the zero with the
 // quotient's sign, as the division would (whose zero case is a slow path).
+// The window test runs beside the correction chain (select and one rarely
+// taken branch at the end), so a dependent chain pays the chain's latency only.
 __device__ __forceinline__ double div(double a, double b, double y) {
-    if (y != 0.0) {
-        if (a == 0.0) return __dmul_rn(a, y);
-        if (in_range(a)) {
-            const double q0 = __dmul_rn(a, y);
-            const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
-            return __fma_rn(__fma_rn(-b, q1, a), y, q1);
-        }
-    }
-    return a / b;
+    const double q0 = __dmul_rn(a, y);
+    const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
+    const double q2 = __fma_rn(__fma_rn(-b, q1, a), y, q1);
+    const bool zero = a == 0.0;
+    if (y == 0.0 || !(zero || in_range(a))) return slow_div(a, b);
+    return zero ? q0 : q2;
 }
 __device__ __forceinline__ float div(float a, float b, float y) {
     if (y != 0.0f) {
