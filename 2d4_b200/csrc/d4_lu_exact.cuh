@@ -231,15 +231,8 @@ __device__ __forceinline__ int src_row(int r, const int *sa, const int *sb, int 
     return r;
 }
 
-// Quotient a / b from y = RN(1/b): the correction chain of d4_qdiv.cuh without
-// its window test.  With b and a inside qdiv's window (or a zero) this is the
-// IEEE quotient; a zero may lose its sign, which no later value depends on.
-__device__ __forceinline__ double quot(double a, double b, double y) {
-    const double q0 = __dmul_rn(a, y);
-    const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
-    return __fma_rn(__fma_rn(-b, q1, a), y, q1);
-}
-__device__ __forceinline__ bool quot_ok(double a) { return qdiv::in_range(a) || a == 0.0; }
+// A numerator of qdiv::fast whose divisor's reciprocal is known to be in window.
+__device__ __forceinline__ bool value_ok(double a) { return qdiv::in_range(a) | (a == 0.0); }
 
 // Reciprocal estimate (relative error about 2^-20), the seed of Newton steps.
 __device__ __forceinline__ double rcp_seed(double d) {
@@ -337,9 +330,9 @@ __device__ __forceinline__ unsigned eliminate(double (&c)[4], bool &bad) {
         double dn = 0.0, yn = 0.0;
         if (i < 3) {
             yn = rcp_seed(__fma_rn(-__dmul_rn(a10, y), u[in], a11));
-            dn = a11 - quot(a10, d, y) * u[in];
+            dn = a11 - qdiv::fast(a10, d, y) * u[in];
         }
-        const double l = quot(v, d, y);
+        const double l = qdiv::fast(v, d, y);
         const bool low = lane > k;
         const double lz = low ? l : 0.0;
         S.lcol[k][lane] = lz;
@@ -360,7 +353,7 @@ __device__ __forceinline__ unsigned eliminate(double (&c)[4], bool &bad) {
         S.s[lane][k0 + i] = c[i];
         S.q[lane][k0 + i] = pre[i];
         if (lane == 0) S.rs[k0 + i] = ys[i];
-        good = good && recip_ok(piv[i], e2s[i]) && (!low || quot_ok(pre[i]));
+        good = good && recip_ok(piv[i], e2s[i]) && (!low || value_ok(pre[i]));
         if (low && fabs(c[i]) > 1.0) msk |= 1u << (k0 + i);
     }
     bad = !good;
@@ -520,7 +513,7 @@ __device__ __forceinline__ bool row_core(double (&c)[kHold], double (&pre)[kHold
             const int k = kLanes * s + own, s1 = s < kHold - 1 ? s + 1 : s;
             const double vn = own < kLanes - 1 ? __shfl_sync(0xffffffffu, c[s], gb + own + 1)
                                                : __shfl_sync(0xffffffffu, c[s1], gb);
-            const double l = quot(v, S.s[k][k], S.rs[k]);
+            const double l = qdiv::fast(v, S.s[k][k], S.rs[k]);
             if (q == own) pre[s] = v;
             v = vn - l * S.s[k][k < 31 ? k + 1 : 31];
             const double cs = c[s] - l * S.s[k][q + kLanes * s];
@@ -530,7 +523,7 @@ __device__ __forceinline__ bool row_core(double (&c)[kHold], double (&pre)[kHold
         }
     }
 #pragma unroll
-    for (int t = 0; t < kHold; ++t) good = good && quot_ok(pre[t]);
+    for (int t = 0; t < kHold; ++t) good = good && value_ok(pre[t]);
     return __all_sync(0xffffffffu, good);
 }
 

@@ -35,29 +35,35 @@ __device__ __forceinline__ T recip(T b) {
     return in_range(b) ? T(1) / b : T(0);
 }
 
-// The division itself, out of line: taken outside the window only.
-static __device__ __noinline__ double slow_div(double a, double b) { return a / b; }
-
-// A zero numerator over an in-window divisor gives a y: the zero with the
-// quotient's sign, as the division would (whose zero case is a slow path).
-// The window test runs beside the correction chain (select and one rarely
-// taken branch at the end), so a dependent chain pays the chain's latency only.
-__device__ __forceinline__ double div(double a, double b, double y) {
+// a / b from y = recip(b) without the window test: the IEEE quotient when
+// fast_ok(a, y), except that a zero may lose its sign (no later value depends on
+// it: solutions and factors are compared and used by value).  For dependent
+// chains, whose caller tests the window beside the chain and redoes the few
+// values that leave it with the division itself; a branch around each quotient
+// more than doubled a substitution's row.
+__device__ __forceinline__ double fast(double a, double b, double y) {
     const double q0 = __dmul_rn(a, y);
     const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
-    const double q2 = __fma_rn(__fma_rn(-b, q1, a), y, q1);
-    const bool zero = a == 0.0;
-    if (y == 0.0 || !(zero || in_range(a))) return slow_div(a, b);
-    return zero ? q0 : q2;
+    return __fma_rn(__fma_rn(-b, q1, a), y, q1);
 }
-__device__ __forceinline__ float div(float a, float b, float y) {
-    if (y != 0.0f) {
-        if (a == 0.0f) return __fmul_rn(a, y);
-        if (in_range(a)) {
-            const float q0 = __fmul_rn(a, y);
-            const float q1 = __fmaf_rn(__fmaf_rn(-b, q0, a), y, q0);
-            return __fmaf_rn(__fmaf_rn(-b, q1, a), y, q1);
-        }
+__device__ __forceinline__ float fast(float a, float b, float y) {
+    const float q0 = __fmul_rn(a, y);
+    const float q1 = __fmaf_rn(__fmaf_rn(-b, q0, a), y, q0);
+    return __fmaf_rn(__fmaf_rn(-b, q1, a), y, q1);
+}
+template <typename T>
+__device__ __forceinline__ bool fast_ok(T a, T y) {
+    return (in_range(a) | (a == T(0))) & (y != T(0));
+}
+
+// The IEEE quotient of one value.  A zero numerator over an in-window divisor
+// gives a y: the zero with the quotient's sign, as the division would (whose
+// zero case is a slow path).
+template <typename T>
+__device__ __forceinline__ T div(T a, T b, T y) {
+    if (y != T(0)) {
+        if (a == T(0)) return a * y;
+        if (in_range(a)) return fast(a, b, y);
     }
     return a / b;
 }

@@ -47,24 +47,29 @@ constexpr long long kSpinLimit = 1ll << 25;  // polls: > 1 s
 // exact order; float: the mixed form, inside refinement), by one thread-block
 // cluster of kClusterCtas CTAs, one warp per 32-row block: block b belongs to
 // warp b / C of CTA b % C (a warp takes further blocks b + C * warps when there
-// are more blocks than warps).  A warp copies its diagonal tile into its shared
-// slot when it starts the block, loads each off-diagonal factor tile straight
-// into registers before it waits for that tile's x values (the load overlaps
-// the wait), applies the tile, then solves its diagonal block.  A finished
-// block's 32 values are pushed into EVERY CTA's shared copy of x with
-// asynchronous stores (st.async ... mbarrier::complete_tx) that count down the
-// transaction bytes which that CTA's mbarrier for the block expects; a consumer
-// waits on its own barrier (acquire) and reads the values locally.  The
-// hand-off is one distributed-shared-memory store per value, with no fence and
-// no flag poll.  Each entry receives its updates in the oracle's order
-// (forward: k ascending; backward: k descending, then the division; updates
-// with a zero value skipped), so the result is bit-identical to the sequential
-// substitution.  Waits are bounded: after kSpinLimit polls a warp records
-// err[0] and stops waiting (the host then discards the results); all CTAs meet
-// at a final cluster barrier, so none exits while another may still write into
-// its shared memory.
+// are more blocks than warps).  A warp streams its block's factor tiles, the
+// diagonal one last, through two shared-memory stages (cp.async: the next tile
+// loads while the current one waits for its x values and is applied; loaded only
+// after the previous tile was applied, each tile's memory latency stood in the
+// chain of the blocks), then solves its diagonal block.  Every lane forms
+// every x value of the block itself, from the right-hand side broadcast a step
+// early, so the chain of a row is one product and difference (and the quotient
+// where it divides) without a shuffle.  After each 8 rows the values go to every
+// CTA's shared copy of x by asynchronous stores (st.async ...
+// mbarrier::complete_tx) that count down the bytes which that CTA's mbarrier for
+// the 8-row group expects.  A consumer waits on its own barrier (acquire) group by group, so it applies a
+// block's first values while the last ones are still being formed.  With one
+// shuffle per row in the chain, whole blocks handed over and a window branch
+// around each quotient a row took 130 (forward) and 300 cycles (backward).  Each
+// entry receives its updates in the oracle's order (forward: k ascending;
+// backward: k descending, then the division), so the result equals the
+// sequential substitution's.  (The oracle skips updates with a zero value; here
+// they are applied: x - l*0 == x.)  Waits are bounded: after kSpinLimit polls a
+// warp records err[0] and stops waiting (the host then discards the results);
+// all CTAs meet at a final cluster barrier, so none exits while another may
+// still write into its shared memory.
 constexpr int kClusterCtas = 8;
-constexpr int kClusterMaxWarps = 16;
+constexpr int kClusterMaxWarps = 8;
 
 __device__ __forceinline__ unsigned cluster_rank() {
     unsigned r;
@@ -86,18 +91,18 @@ __device__ __forceinline__ uint32_t mapa(uint32_t addr, unsigned cta) {
     return r;
 }
 // Asynchronous store into another CTA's shared memory that completes
-// sizeof(v) bytes of the transaction count of that CTA's mbarrier `mbar`.
+// sizeof(v) bytes of the transaction count of that CTA's mbarrier `mbar`.  No
+// memory clobber: it orders nothing of this thread's, and would keep the chain's
+// shared-memory operands from being loaded ahead.
 __device__ __forceinline__ void st_async(uint32_t addr, double v, uint32_t mbar) {
     asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];" ::"r"(
                      addr),
-                 "d"(v), "r"(mbar)
-                 : "memory");
+                 "d"(v), "r"(mbar));
 }
 __device__ __forceinline__ void st_async(uint32_t addr, float v, uint32_t mbar) {
     asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(
                      addr),
-                 "f"(v), "r"(mbar)
-                 : "memory");
+                 "f"(v), "r"(mbar));
 }
 __device__ __forceinline__ void arrive_expect_tx(uint32_t mbar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes)
@@ -121,26 +126,37 @@ __host__ __device__ constexpr int cluster_warps(int n) {
                : kClusterMaxWarps;
 }
 
-// x (n values), one mbarrier per 32-row block, and a 32 x 33 diagonal-tile
-// slot per warp.
+// x (n values), four mbarriers (8-row groups) per 32-row block, and per warp two
+// 32 x 32 tile stages and the diagonal's reciprocals.
 template <typename T>
 __host__ __device__ constexpr size_t cluster_smem_bytes(int n) {
-    return ((sizeof(T) * (size_t)n + 15) / 16) * 16 +
-           ((8 * (size_t)((n + 31) / 32) + 15) / 16) * 16 +
-           sizeof(T) * 32 * 33 * (size_t)kClusterMaxWarps;
+    return ((sizeof(T) * (size_t)n + 15) / 16) * 16 + 32 * (size_t)((n + 31) / 32) +
+           sizeof(T) * (2 * 32 * 32 + 32) * (size_t)kClusterMaxWarps;
 }
 
-// Tile (row block b, column block kb) of the factors into registers: lane l
-// gets row 32 b + l, columns 32 kb .. 32 kb + 31.
+// Tile (row block b, column block kb) of the factors into st[column][row] by one
+// warp, asynchronously (element pairs; n is even, so pairs never straddle the
+// edge, past which the tile is zero).
 template <typename T>
-__device__ __forceinline__ void tile_regs(const T *__restrict__ LU, int n, int b, int kb, int lane,
-                                          T (&t)[32]) {
-    const int r = b * 32 + lane;
+__device__ __forceinline__ void tile_async(const T *__restrict__ LU, int n, int b, int kb, int lane,
+                                           T (*st)[32]) {
+    const int r = 2 * (lane & 15), row = b * 32 + r;
 #pragma unroll
-    for (int k = 0; k < 32; ++k) {
-        const int cidx = kb * 32 + k;
-        t[k] = (r < n && cidx < n) ? LU[(size_t)r + (size_t)cidx * n] : T(0);
+    for (int i = 0; i < 16; ++i) {
+        const int k = 2 * i + (lane >> 4), col = kb * 32 + k;
+        const bool ok = row < n && col < n;
+        const T *src = ok ? LU + (size_t)row + (size_t)col * n : LU;
+        const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(&st[k][r]));
+        if (sizeof(T) == 8)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src),
+                         "r"(ok ? 16 : 0)
+                         : "memory");
+        else
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src),
+                         "r"(ok ? 8 : 0)
+                         : "memory");
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
 // kTrans: the factors are given transposed (Lt = (LU)^T) and the system is
@@ -155,22 +171,29 @@ __global__ void __launch_bounds__(32 * kClusterMaxWarps) k_trsv_cluster(
     const int nblk = (n + 31) / 32;
     T *xall = reinterpret_cast<T *>(craw);
     uint64_t *mbar = reinterpret_cast<uint64_t *>(craw + ((sizeof(T) * (size_t)n + 15) / 16) * 16);
-    T(*dslot)[32][33] = reinterpret_cast<T(*)[32][33]>(reinterpret_cast<unsigned char *>(mbar) +
-                                                      ((8 * (size_t)nblk + 15) / 16) * 16);
+    T *slot = reinterpret_cast<T *>(mbar + 4 * (size_t)nblk);
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
     const int C = (int)cluster_size(), c = (int)cluster_rank();
-    // one barrier per block, expecting the block's values (kw x sizeof(T)
-    // bytes) from its producer's asynchronous stores
-    for (int b = tid; b < nblk; b += blockDim.x) {
+    // one barrier per 8-row group, expecting the group's values from their
+    // producer's asynchronous stores
+    for (int b = tid; b < 4 * nblk; b += blockDim.x) {
         const uint32_t ma = static_cast<uint32_t>(__cvta_generic_to_shared(mbar + b));
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(ma) : "memory");
-        arrive_expect_tx(ma, (uint32_t)(sizeof(T) * min(32, n - b * 32)));
+        if (b * 8 < n) arrive_expect_tx(ma, (uint32_t)(sizeof(T) * min(8, n - b * 8)));
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncthreads();
     cluster_sync_all();
     bool aborted = false;
-    T(*dt)[33] = dslot[w];
+    slot += w * (2 * 32 * 32 + 32);
+    T(*stage)[32][32] = reinterpret_cast<T(*)[32][32]>(slot);
+    T *rec = slot + 2 * 32 * 32;
+    // the CTAs this lane sends to
+    const uint32_t xa = static_cast<uint32_t>(__cvta_generic_to_shared(xall));
+    const uint32_t ma0 = static_cast<uint32_t>(__cvta_generic_to_shared(mbar));
+    const unsigned p0 = min(lane >> 3, C - 1), p1 = min((lane >> 3) + 4, C - 1);
+    const uint32_t xpeer0 = mapa(xa, p0), mpeer0 = mapa(ma0, p0);
+    const uint32_t xpeer1 = mapa(xa, p1), mpeer1 = mapa(ma0, p1);
     // this warp's blocks, in solve order
     const int first = c + C * w, stride = C * nw;
     const int nmine = first < nblk ? (nblk - 1 - first) / stride + 1 : 0;
@@ -179,78 +202,123 @@ __global__ void __launch_bounds__(32 * kClusterMaxWarps) k_trsv_cluster(
         const int row = b * 32 + lane;
         const bool row_ok = row < n;
         T xi = row_ok ? (kFwd ? T(kTrans ? ga.g_in[row] : g_of(ga, perm[row])) : xin[row]) : T(0);
-        T tl[32];
-        // the diagonal tile, early, into this warp's shared slot (row per lane)
-        tile_regs(LU, n, b, b, lane, tl);
-#pragma unroll
-        for (int k = 0; k < 32; ++k) dt[lane][k] = tl[k];
-        __syncwarp();
-        // this lane's divisor and its reciprocal, formed before the chain
-        // (the quotient in the chain is still the IEEE one)
-        const T dmine = dt[lane][lane];
-        const T rmine = qdiv::recip(dmine);
         const int napply = kFwd ? b : nblk - 1 - b;
+        tile_async(LU, n, b, napply > 0 ? (kFwd ? 0 : nblk - 1) : b, lane, stage[0]);
+        // the diagonal's reciprocals, formed before the chain (the quotient in
+        // the chain is still the IEEE one; rows past the matrix are an identity's)
+        rec[lane] = row_ok ? qdiv::recip(LU[(size_t)row + (size_t)row * n]) : T(1);
         for (int s = 0; s < napply; ++s) {
             const int kb = kFwd ? s : nblk - 1 - s;
             const int kw = min(32, n - kb * 32);
-            tile_regs(LU, n, b, kb, lane, tl);
-            if (!aborted) {
-                const uint32_t ma = static_cast<uint32_t>(__cvta_generic_to_shared(mbar + kb));
-                long long spins = 0;
-                bool ok = true;
-                while (!try_wait_cluster(ma)) {
-                    if (++spins > kSpinLimit) {
-                        ok = false;
-                        break;
-                    }
-                }
-                if (!__all_sync(0xffffffffu, ok)) {
-                    aborted = true;
-                    if (lane == 0 && atomicCAS(err, 0, 1) == 0) {
-                        err[1] = b;
-                        err[2] = kb;
-                        err[3] = -1;
-                        err[4] = -1;
-                    }
-                }
-            }
+            tile_async(LU, n, b, kFwd ? s + 1 : nblk - 2 - s, lane, stage[(s + 1) & 1]);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncwarp();
+            const T(*tl)[32] = stage[s & 1];
             const T *xb = xall + kb * 32;
-            if (kFwd) {
 #pragma unroll
-                for (int k = 0; k < 32; ++k) {
-                    const T t = xb[k < kw ? k : 0];
-                    if (k < kw && t != T(0)) xi = xi - tl[k] * t;
-                }
-            } else {
+            for (int gq = 0; gq < 4; ++gq) {
+                const int g = kFwd ? gq : 3 - gq;
+                if (g * 8 >= kw) continue;
+                T l8[8];
 #pragma unroll
-                for (int k = 31; k >= 0; --k) {
-                    const T t = xb[k < kw ? k : 0];
-                    if (k < kw && t != T(0)) xi = xi - tl[k] * t;
+                for (int e = 0; e < 8; ++e) l8[e] = tl[8 * g + e][lane];
+                if (!aborted) {
+                    const uint32_t ma =
+                        static_cast<uint32_t>(__cvta_generic_to_shared(mbar + kb * 4 + g));
+                    long long spins = 0;
+                    bool ok = true;
+                    while (!try_wait_cluster(ma)) {
+                        if (++spins > kSpinLimit) {
+                            ok = false;
+                            break;
+                        }
+                    }
+                    if (!__all_sync(0xffffffffu, ok)) {
+                        aborted = true;
+                        if (lane == 0 && atomicCAS(err, 0, 1) == 0) {
+                            err[1] = b;
+                            err[2] = kb;
+                            err[3] = -1;
+                            err[4] = -1;
+                        }
+                    }
                 }
+                if (kw == 32) {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        const int k = kFwd ? 8 * g + e : 8 * g + 7 - e;
+                        xi = xi - l8[k & 7] * xb[k];
+                    }
+                } else {
+                    // the last block's: no product with what lies past it
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        const int k = kFwd ? 8 * g + e : 8 * g + 7 - e;
+                        if (k < kw) xi = xi - l8[k & 7] * xb[k];
+                    }
+                }
+            }
+            __syncwarp();  // this stage is free for the tile after next
+        }
+        // diagonal block, 8 rows at a time: v is row k's right-hand side, then its
+        // x value
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncwarp();
+        T(*dt)[32] = stage[napply & 1];  // [column][row]
+        if (!row_ok) dt[lane][lane] = T(1);
+        __syncwarp();
+        constexpr bool kDivides = kFwd == kTrans;
+#pragma unroll 1
+        for (int gq = 0; gq < 4; ++gq) {
+            const int g8 = kFwd ? 8 * gq : 24 - 8 * gq;
+            // where it divides, the chain's operands first (930 against 1000 cycles
+            // a group; without the division the compiler's order is the better one)
+            T own[8], nxt[8], dd[8], rr[8];
+            if (kDivides) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const int k = kFwd ? g8 + e : g8 + 7 - e, kn = (kFwd ? k + 1 : k - 1) & 31;
+                    own[e] = dt[k][lane];
+                    nxt[e] = dt[k][kn];
+                    dd[e] = dt[k][k];
+                    rr[e] = rec[k];
+                }
+            }
+            const T x0 = xi;
+            T v = __shfl_sync(0xffffffffu, xi, kFwd ? g8 : g8 + 7), pre = T(0);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const int k = kFwd ? g8 + e : g8 + 7 - e, kn = (kFwd ? k + 1 : k - 1) & 31;
+                const T vn = __shfl_sync(0xffffffffu, xi, kn);
+                if (kDivides) {
+                    if (lane == k) pre = v;
+                    v = qdiv::fast(v, dd[e], rr[e]);
+                }
+                const T t = xi - (kDivides ? own[e] : dt[k][lane]) * v;
+                xi = lane == k ? v : ((kFwd ? lane > k : lane < k) ? t : xi);
+                v = vn - (kDivides ? nxt[e] : dt[k][kn]) * v;
+            }
+            if (kDivides && !__all_sync(0xffffffffu, qdiv::fast_ok(pre, rec[lane]))) {
+                // outside the quotient window: the same rows with the division
+                xi = x0;
+#pragma unroll 1
+                for (int e = 0; e < 8; ++e) {
+                    const int k = kFwd ? g8 + e : g8 + 7 - e;
+                    const T x = __shfl_sync(0xffffffffu, xi, k) / dt[k][k];
+                    const T t = xi - dt[k][lane] * x;
+                    xi = lane == k ? x : ((kFwd ? lane > k : lane < k) ? t : xi);
+                }
+            }
+            // lane l sends row l % 8 of the group to CTAs l / 8 and l / 8 + 4
+            const int r = b * 32 + g8 + (lane & 7);
+            const T x = __shfl_sync(0xffffffffu, xi, g8 + (lane & 7));
+            if (r < n) {
+                const uint32_t xo = (uint32_t)(r * sizeof(T)), mo = (uint32_t)((r >> 3) * 8);
+                if ((lane >> 3) < C) st_async(xpeer0 + xo, x, mpeer0 + mo);
+                if ((lane >> 3) + 4 < C) st_async(xpeer1 + xo, x, mpeer1 + mo);
             }
         }
-        // diagonal block
-        const int kw = min(32, n - b * 32);
-        if (kFwd) {
-#pragma unroll
-            for (int k = 0; k < 32; ++k) {
-                if (kTrans && k < kw && lane == k) xi = qdiv::div(xi, dmine, rmine);
-                const T t = __shfl_sync(0xffffffffu, xi, k);
-                if (k < kw && lane > k && t != T(0)) xi = xi - dt[lane][k] * t;
-            }
-        } else {
-#pragma unroll
-            for (int k = 31; k >= 0; --k) {
-                if (!kTrans && k < kw && lane == k) xi = qdiv::div(xi, dmine, rmine);
-                const T t = __shfl_sync(0xffffffffu, xi, k);
-                if (k < kw && lane < k && t != T(0)) xi = xi - dt[lane][k] * t;
-            }
-        }
-        // push to every CTA: asynchronous stores completing that CTA's barrier
-        const uint32_t xa = static_cast<uint32_t>(__cvta_generic_to_shared(xall + b * 32 + lane));
-        const uint32_t mba = static_cast<uint32_t>(__cvta_generic_to_shared(mbar + b));
-        if (row_ok)
-            for (int q = 0; q < C; ++q) st_async(mapa(xa, (unsigned)q), xi, mapa(mba, (unsigned)q));
+        __syncwarp();
         if (row_ok) {
             xg[(kTrans && !kFwd) ? perm[row] : row] = xi;
             if (!kFwd && !kTrans) {
