@@ -10,15 +10,15 @@
 //                  instance by a prefix table), the same tile body as the
 //                  single-system engine (d4_sweep64.cuh);
 //   row sums       all instances' 32-row blocks in one grid (same pipeline);
-//   LU, solves     one CTA per instance: an exact-order blocked LU (panel of
-//                  32 columns, U12 by column, trailing update in 64x64 tiles
-//                  from shared memory) and column-oriented substitutions,
-//                  each entry receiving its updates in the oracle's order, so
-//                  every instance reproduces the single-system result bit
-//                  for bit;
+//   LU             one thread-block cluster per instance, running the
+//                  single-system engine's exact-order LU (d4_lu_exact.cuh)
+//                  with the cluster as its group of CTAs;
+//   solves         one CTA per instance, the single-system engine's blocked
+//                  substitutions (d4_trsv.cuh), so every instance reproduces
+//                  the single-system result bit for bit;
 //   elementwise    one CTA per instance, or a prefix table for n^2 work.
-// Instances are ordered by decreasing n, so the largest (whose one-CTA LU is
-// the longest) start first.  After each round the host applies each
+// Instances are ordered by decreasing n, so the largest (whose LU is the
+// longest) start first.  After each round the host applies each
 // instance's step control exactly as d4_run does (acceptance, new step size,
 // limits), and the next round's per-instance scalars are uploaded in one copy.
 #include <algorithm>
@@ -28,13 +28,16 @@
 #include <string>
 #include <vector>
 
+#include "d4_lu_exact.cuh"
 #include "d4_sweep64.cuh"
+#include "d4_trsv.cuh"
 
 namespace d4 {
 namespace ens {
 
 enum Vec {
     kX0, kY, kXB, kXH, kX2, kVI, kVI2, kSP, kSP2, kDV, kDVN, kFAC, kTOL, kRSUB, kRSC,
+    kW1, kW2,  // the solves' forward and backward results
     kNumVec
 };
 
@@ -43,6 +46,7 @@ struct Inst {
     int pad;
     long long voff;  // offset of the instance's vectors in every vector pool
     long long moff;  // offset of its n x n matrices in every matrix pool
+    long long woff;  // offset of its LU schedule words
     double cutoff, cut_sq, one_per_cut_sq;
 };
 
@@ -57,13 +61,16 @@ struct Sc {
 struct Pools {
     double *v[kNumVec];
     double *F, *A, *LU;
-    int *piv;
-    int *sing;        // per instance: the current factorisation met a zero pivot
-    int *sing_any;    // per instance: some factorisation of the round did
+    int *piv, *perm;
+    double *lu_p0, *lu_q, *lu_u, *lu_dg;  // the LU's buffers (voff x 32, 64, 64; per instance)
+    unsigned *lu_words;                   // its mask and schedule words
+    LuMaps *lu_maps;                      // per instance
+    int *lu_flags;    // per instance kFlagCount words of the current factorisation
+    int *sing_any;    // per instance: some factorisation of the round met a zero pivot
     double *ratio;    // per instance: {max err^2/tol, index}
     double *strain;   // per instance: accumulated strain
     int *acc;         // per instance: accepted this round
-    int *err;         // row-pipeline wait failure
+    int *err;         // wait failures: [0] row pipeline, [1] LU, [2..6] solves
 };
 
 struct Common {
@@ -191,265 +198,85 @@ __global__ void k_ens_half_finish(Pools P, const Inst *ins, const Sc *sc, const 
     }
 }
 
-// ---- one-CTA exact-order LU -------------------------------------------------
-constexpr int kLuT = 256;
-constexpr int kPan = 32;
-constexpr int kTt = 64;  // trailing tile edge
-
-__device__ __forceinline__ void argmax_combine(double &v, int &i, double ov, int oi) {
-    if (oi >= 0 && (ov > v || (ov == v && (i < 0 || oi < i)))) {
-        v = ov;
-        i = oi;
+// Copies the instance's A into LU and factorises it there, by one cluster per
+// instance.  The cluster takes the place of the grid of the single-system LU:
+// its barriers are the hardware's, and a large instance's LU is spread over
+// several SMs (one CTA per instance took 168 ms for n = 2048, the length of the
+// whole round's factorisation; a cluster of 4 takes 20 ms).
+__global__ void __launch_bounds__(lux::kThreads, 1) k_ens_lu(Pools P, const Inst *ins,
+                                                             const int *act) {
+    lux::ClusterGroup g;
+    const int G = g.size(), cta = g.rank();
+    const int k = act[blockIdx.x / G];
+    const Inst in = ins[k];
+    const int n = in.n;
+    lux::Args a;
+    a.n = n;
+    a.A = P.LU + in.moff;
+    a.P0 = P.lu_p0 + in.voff * lux::NB;
+    a.Q = P.lu_q + in.voff * 2 * lux::NB;
+    a.U = P.lu_u + in.voff * 2 * lux::NB;
+    a.dg = P.lu_dg + (size_t)k * lux::kDgWords;
+    a.mask = P.lu_words + in.woff;
+    a.sched = a.mask + lu_pass_words((n + lux::NB - 1) / lux::NB);
+    a.perm = P.perm + in.voff;
+    a.piv = P.piv + in.voff;
+    a.flags = P.lu_flags + k * kFlagCount;
+    a.map_a = &P.lu_maps[k].a;
+    a.map_u = &P.lu_maps[k].u;
+    if (threadIdx.x == 0) {
+        // tensor maps in global memory: acquired by the thread that uses them
+        asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(a.map_a)
+                     : "memory");
+        asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(a.map_u)
+                     : "memory");
+    }
+    const double2 *src = reinterpret_cast<const double2 *>(P.A + in.moff);
+    double2 *dst = reinterpret_cast<double2 *>(a.A);
+    const size_t total = (size_t)n * n / 2, step = (size_t)G * lux::kThreads;
+    size_t i = (size_t)cta * lux::kThreads + threadIdx.x;
+    for (; i + 7 * step < total; i += 8 * step) {
+        double2 v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = src[i + e * step];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) dst[i + e * step] = v[e];
+    }
+    for (; i < total; i += step) dst[i] = src[i];
+    g.arrive(false);
+    g.wait(nullptr, a.flags);
+    lux::factor(a, g);
+    if (cta == 0 && threadIdx.x == 0) {
+        if (a.flags[kFlagSingular]) P.sing_any[k] = 1;
+        if (a.flags[kFlagBarrierTimeout]) atomicOr(P.err + 1, 1);
     }
 }
 
-// Factorises the instance's A into LU with the operation sequence of the
-// oracle's partial-pivot LU (first maximum wins, whole-row swaps, column
-// divided by the pivot, each entry updated k ascending with the product and
-// the difference rounded separately, and updates with u_kj == 0 skipped).
-__global__ void __launch_bounds__(kLuT) k_ens_lu(Pools P, const Inst *ins, const int *act) {
-    __shared__ double sL[kTt][kPan + 1];
-    __shared__ double sU[kPan][kTt + 1];
-    __shared__ double rv[kLuT / 32];
-    __shared__ int ri[kLuT / 32];
-    __shared__ int s_piv;
-    __shared__ double prow[kPan];
+// Both substitutions of one solve, residual and update included, by one CTA per
+// instance (the blocked solve of d4_trsv.cuh, its warps handing the values over
+// within the CTA).
+__global__ void __launch_bounds__(32 * trsv::kClusterMaxWarps)
+    k_ens_solve(Pools P, const Inst *ins, const Sc *sc, const int *act, int gmode, double hmul,
+                int se, int si, int xn, int xo, int base, int out) {
     const int k = act[blockIdx.x];
     const Inst in = ins[k];
-    const int n = in.n, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    double *a = P.LU + in.moff;
-    const double *a0 = P.A + in.moff;
-    int *piv = P.piv + in.voff;
-    const size_t nn = (size_t)n * n;
-    for (size_t idx = tid; idx < nn; idx += kLuT) a[idx] = a0[idx];
-    __syncthreads();
-    int singular = 0;
-    for (int k0 = 0; k0 < n; k0 += kPan) {
-        const int kw = min(kPan, n - k0);
-        // panel: columns k0 .. k0 + kw - 1, unblocked
-        for (int kk = k0; kk < k0 + kw; ++kk) {
-            const double akk = fabs(a[kk + (size_t)kk * n]);
-            double bv = -1;
-            int bi = -1;
-#pragma unroll 4
-            for (int i = kk + 1 + tid; i < n; i += kLuT) {
-                const double v = fabs(a[i + (size_t)kk * n]);
-                if (v > bv) {
-                    bv = v;
-                    bi = i;
-                }
-            }
-            for (int o = 16; o > 0; o >>= 1) {
-                const double ov = __shfl_down_sync(0xffffffffu, bv, o);
-                const int oi = __shfl_down_sync(0xffffffffu, bi, o);
-                argmax_combine(bv, bi, ov, oi);
-            }
-            if (lane == 0) {
-                rv[wid] = bv;
-                ri[wid] = bi;
-            }
-            __syncthreads();
-            if (tid == 0) {
-                double v = rv[0];
-                int i = ri[0];
-                for (int w = 1; w < kLuT / 32; ++w) argmax_combine(v, i, rv[w], ri[w]);
-                // the sequential scan starts from |a_kk| and replaces only on a
-                // strictly greater value (a NaN |a_kk| is never replaced)
-                s_piv = (i >= 0 && v > akk) ? i : kk;
-                piv[kk] = s_piv;
-            }
-            __syncthreads();
-            const int p = s_piv;
-            if (a[p + (size_t)kk * n] == 0.0) {
-                singular = 1;
-                __syncthreads();
-                continue;
-            }
-            if (p != kk)
-                for (int j = tid; j < n; j += kLuT) {
-                    const double t = a[kk + (size_t)j * n];
-                    a[kk + (size_t)j * n] = a[p + (size_t)j * n];
-                    a[p + (size_t)j * n] = t;
-                }
-            __syncthreads();
-            const double d = a[kk + (size_t)kk * n];
-#pragma unroll 4
-            for (int i = kk + 1 + tid; i < n; i += kLuT) a[i + (size_t)kk * n] /= d;
-            __syncthreads();
-            // rank-1 update of the panel's remaining columns: a thread per row,
-            // the row's loads issued together (one memory round trip per row)
-            const int ncol = k0 + kw - kk - 1;
-            if (tid < kPan) prow[tid] = tid < ncol ? a[kk + (size_t)(kk + 1 + tid) * n] : 0.0;
-            __syncthreads();
-            for (int i = kk + 1 + tid; i < n; i += kLuT) {
-                const double l = a[i + (size_t)kk * n];
-                double v[kPan - 1];
-#pragma unroll
-                for (int q = 0; q < kPan - 1; ++q)
-                    v[q] = q < ncol ? a[i + (size_t)(kk + 1 + q) * n] : 0.0;
-#pragma unroll
-                for (int q = 0; q < kPan - 1; ++q) {
-                    const double t = prow[q];
-                    if (q < ncol && t != 0.0) a[i + (size_t)(kk + 1 + q) * n] = v[q] - l * t;
-                }
-            }
-            __syncthreads();
-        }
-        const int j1 = k0 + kw;
-        if (j1 >= n) break;
-        // U12: rows k0 .. k0 + kw - 1 of columns j >= j1 (unit lower L11 from sL)
-        for (int t = tid; t < kPan * kPan; t += kLuT) {
-            const int r = t % kPan, c = t / kPan;
-            sL[r][c] = (r < kw && c < kw) ? a[(k0 + r) + (size_t)(k0 + c) * n] : 0.0;
-        }
-        __syncthreads();
-        for (int j = j1 + tid; j < n; j += kLuT) {
-            double u[kPan];
-            double *col = a + k0 + (size_t)j * n;
-#pragma unroll
-            for (int r = 0; r < kPan; ++r) u[r] = r < kw ? col[r] : 0.0;
-#pragma unroll
-            for (int c = 0; c < kPan; ++c) {
-                const double t = u[c];
-                if (c < kw && t != 0.0) {
-#pragma unroll
-                    for (int r = c + 1; r < kPan; ++r)
-                        if (r < kw) u[r] -= sL[r][c] * t;
-                }
-            }
-#pragma unroll
-            for (int r = 0; r < kPan; ++r)
-                if (r < kw) col[r] = u[r];
-        }
-        __syncthreads();
-        // trailing update in kTt x kTt tiles: thread (tr, tc) owns rows
-        // i0 + tr + 16 q and columns j0 + tc + 16 w (q, w = 0..3)
-        const int tr = tid & 15, tc = tid >> 4;
-        for (int i0 = j1; i0 < n; i0 += kTt) {
-            for (int jt = j1; jt < n; jt += kTt) {
-                for (int t = tid; t < kTt * kPan; t += kLuT) {
-                    const int r = t % kTt, c = t / kTt;
-                    sL[r][c] = (i0 + r < n && c < kw) ? a[(i0 + r) + (size_t)(k0 + c) * n] : 0.0;
-                }
-                for (int t = tid; t < kTt * kPan; t += kLuT) {
-                    const int r = t % kPan, c = t / kPan;
-                    sU[r][c] = (jt + c < n && r < kw) ? a[(k0 + r) + (size_t)(jt + c) * n] : 0.0;
-                }
-                __syncthreads();
-                double acc[4][4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-#pragma unroll
-                    for (int w = 0; w < 4; ++w) {
-                        const int i = i0 + tr + 16 * q, j = jt + tc + 16 * w;
-                        acc[q][w] = (i < n && j < n) ? a[i + (size_t)j * n] : 0.0;
-                    }
-                for (int c = 0; c < kw; ++c) {
-                    double lv[4], uv[4];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) lv[q] = sL[tr + 16 * q][c];
-#pragma unroll
-                    for (int w = 0; w < 4; ++w) uv[w] = sU[c][tc + 16 * w];
-                    // the oracle skips an update whose u_kj is 0; when no u of
-                    // this warp's columns is 0 (the dense case) the plain
-                    // product-difference is the same and needs no select
-                    const bool nz = uv[0] != 0.0 && uv[1] != 0.0 && uv[2] != 0.0 && uv[3] != 0.0;
-                    if (__all_sync(0xffffffffu, nz)) {
-#pragma unroll
-                        for (int q = 0; q < 4; ++q)
-#pragma unroll
-                            for (int w = 0; w < 4; ++w) acc[q][w] = acc[q][w] - lv[q] * uv[w];
-                    } else {
-#pragma unroll
-                        for (int q = 0; q < 4; ++q)
-#pragma unroll
-                            for (int w = 0; w < 4; ++w) {
-                                const double nv = acc[q][w] - lv[q] * uv[w];
-                                acc[q][w] = uv[w] != 0.0 ? nv : acc[q][w];
-                            }
-                    }
-                }
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-#pragma unroll
-                    for (int w = 0; w < 4; ++w) {
-                        const int i = i0 + tr + 16 * q, j = jt + tc + 16 * w;
-                        if (i < n && j < n) a[i + (size_t)j * n] = acc[q][w];
-                    }
-                __syncthreads();
-            }
-        }
-    }
-    if (tid == 0) {
-        P.sing[k] = singular;
-        P.sing_any[k] |= singular;
-    }
-}
-
-// ---- one-CTA solve with the LU factors (the oracle's substitution order) ----
-constexpr int kSolT = 512;
-
-__global__ void __launch_bounds__(kSolT) k_ens_solve(Pools P, const Inst *ins, const Sc *sc,
-                                                     const int *act, int gmode, double hmul,
-                                                     int se, int si, int xn, int xo, int base,
-                                                     int out) {
-    extern __shared__ double xs[];
-    const int k = act[blockIdx.x];
-    const Inst in = ins[k];
-    const int n = in.n, tid = threadIdx.x;
-    const double *a = P.LU + in.moff;
-    const int *piv = P.piv + in.voff;
-    const double hv = sc[k].h * hmul;
-    const double *dv = P.v[kDV] + in.voff;
-    const double *s_end = P.v[se] + in.voff, *s_init = P.v[si] + in.voff;
-    for (int r = tid; r < n; r += kSolT) {
-        // residual of the stage, src/simulation.cpp:101,123,142,621
-        const double d = dv[r];
-        const double X = (1 + d) * s_end[r] + (1 - d) * s_init[r];
-        double g;
-        if (gmode == kGBig)
-            g = -hv * X / 2;
-        else if (gmode == kGHalf)
-            g = -hv / 2 * X / 2;
-        else
-            g = P.v[xn][in.voff + r] - P.v[xo][in.voff + r] - hv * X / 2;
-        xs[r] = g;
-    }
-    __syncthreads();
-    if (tid == 0)
-        for (int q = 0; q < n; ++q) {
-            const int p = piv[q];
-            if (p != q) {
-                const double t = xs[q];
-                xs[q] = xs[p];
-                xs[p] = t;
-            }
-        }
-    __syncthreads();
-    for (int q = 0; q < n; ++q) {
-        const double t = xs[q];
-        if (t != 0.0) {
-            const double *cq = a + (size_t)q * n;
-            for (int i = q + 1 + tid; i < n; i += kSolT) xs[i] -= cq[i] * t;
-        }
-        __syncthreads();
-    }
-    for (int q = n - 1; q >= 0; --q) {
-        if (tid == 0) xs[q] /= a[q + (size_t)q * n];
-        __syncthreads();
-        const double t = xs[q];
-        if (t != 0.0) {
-            const double *cq = a + (size_t)q * n;
-            for (int i = tid; i < q; i += kSolT) xs[i] -= cq[i] * t;
-        }
-        __syncthreads();
-    }
-    const int singular = P.sing[k];
-    for (int r = tid; r < n; r += kSolT) {
-        double d = xs[r];
-        if (singular && !((-1 < d) && (d < 1))) d = 0;  // src/simulation.cpp:652-657
-        P.v[out][in.voff + r] = P.v[base][in.voff + r] - d;
-    }
+    trsv::GArgs ga{};
+    ga.gmode = gmode;
+    ga.hval = sc[k].h * hmul;
+    ga.dvec = P.v[kDV] + in.voff;
+    ga.s_end = P.v[se] + in.voff;
+    ga.s_init = P.v[si] + in.voff;
+    ga.x_new = P.v[xn] + in.voff;
+    ga.x_old = P.v[xo] + in.voff;
+    ga.base = P.v[base] + in.voff;
+    ga.out = P.v[out] + in.voff;
+    ga.fix_singular = 1;
+    const double *LU = P.LU + in.moff;
+    const int *perm = P.perm + in.voff, *flags = P.lu_flags + k * kFlagCount;
+    double *w1 = P.v[kW1] + in.voff, *w2 = P.v[kW2] + in.voff;
+    trsv::solve_pass<true, double, false>(in.n, LU, perm, flags, ga, w1, nullptr, P.err + 2);
+    trsv::release_barriers(in.n, sizeof(double));
+    trsv::solve_pass<false, double, false>(in.n, LU, perm, flags, ga, w2, w1, P.err + 2);
 }
 
 __global__ void __launch_bounds__(1024) k_ens_error(Pools P, const Inst *ins, const int *act,
@@ -518,8 +345,9 @@ struct Ensemble {
     int *d_act = nullptr, *d_pre_pair = nullptr, *d_pre_row = nullptr, *d_pre_mat = nullptr;
     std::vector<Sc> hsc;
     std::vector<int> act, pre_pair, pre_row, pre_mat;
-    int solve_smem = 0;
-    long long launches = 0;
+    int solve_smem = 0, solve_warps = 0;
+    int sms = 0;
+    long long words = 0;  // LU schedule words of all instances
     long long vtot = 0;  // entries of each per-dislocation vector pool
     int pair_ty = 8;     // threads per pair tile along j (autotuned, first run)
     bool tuned = false;
@@ -617,16 +445,56 @@ void autotune(Ensemble &E) {
     E.tuned = true;
 }
 
+// CTAs per instance of the LU: the smallest power of two that keeps the largest
+// active instance's factorisation within the others' share of the chip,
+// n_max^3 / G <= sum n^3 / SMs (the work is n^3, and a cluster's efficiency
+// hardly depends on its size: n = 1024 takes 11.7, 6.7, 3.2 and 1.7 ms on 1, 2, 4
+// and 8 CTAs), at most 8 (the portable size).
+int lu_cluster(const Ensemble &E) {
+    double sum = 0, top = 0;
+    for (int k : E.act) {
+        const double c = std::pow((double)E.hi[k].n, 3);
+        sum += c;
+        top = std::max(top, c);
+    }
+    int g = 1;
+    while (g < 8 && g * sum < top * E.sms) g *= 2;
+    return g;
+}
+
+// One cluster of G CTAs per active instance (the kernels use cluster barriers and
+// asynchronous shared stores, so G = 1 is a cluster launch too).
+template <class... Params, class... Values>
+void launch_clusters(Ensemble &E, void (*kernel)(Params...), int G, int threads, int smem,
+                     Values... values) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)E.act.size() * G);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = E.stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = G;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    D4_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, values...));
+}
+
 void lu(Ensemble &E) {
-    k_ens_lu<<<(int)E.act.size(), kLuT, 0, E.stream>>>(E.P, E.d_ins, E.d_act);
+    D4_CUDA_OK(cudaMemsetAsync(E.P.lu_words, 0, sizeof(unsigned) * E.words, E.stream));
+    D4_CUDA_OK(cudaMemsetAsync(E.P.lu_flags, 0, sizeof(int) * kFlagCount * E.count, E.stream));
+    launch_clusters(E, k_ens_lu, lu_cluster(E), lux::kThreads, (int)sizeof(lux::Smem), E.P,
+                    (const Inst *)E.d_ins, (const int *)E.d_act);
     check("k_ens_lu");
 }
 
 void solve(Ensemble &E, int gmode, double hmul, int se, int si, int xn, int xo, int base,
            int out) {
-    k_ens_solve<<<(int)E.act.size(), kSolT, E.solve_smem, E.stream>>>(
-        E.P, E.d_ins, E.d_sc, E.d_act, gmode, hmul, se, si, xn < 0 ? 0 : xn, xo < 0 ? 0 : xo,
-        base, out);
+    launch_clusters(E, k_ens_solve, 1, 32 * E.solve_warps, E.solve_smem, E.P,
+                    (const Inst *)E.d_ins, (const Sc *)E.d_sc, (const int *)E.d_act, gmode, hmul,
+                    se, si, xn < 0 ? 0 : xn, xo < 0 ? 0 : xo, base, out);
     check("k_ens_solve");
 }
 
@@ -708,7 +576,7 @@ int d4_ensemble_create(void **out, int count, const int *n, const d4_params *p) 
         E->cm.heaviside = p->heaviside_cutoff;
         E->cm.wfn = p->weight_function;
         E->cm.calc_strain = p->calculate_strain;
-        long long voff = 0, moff = 0, smax = 0;
+        long long voff = 0, moff = 0, woff = 0, smax = 0;
         E->hi.resize(count);
         E->hins.resize(count);
         for (int k = 0; k < count; ++k) {
@@ -721,6 +589,7 @@ int d4_ensemble_create(void **out, int count, const int *n, const d4_params *p) 
             in.pad = 0;
             in.voff = voff;
             in.moff = moff;
+            in.woff = woff;
             double mult = p->cutoff_multiplier;
             if (!p->heaviside_cutoff && p->cutoff_multiplier >= std::sqrt(2 * (double)n[k]) / 12)
                 mult = 1e20;
@@ -730,9 +599,12 @@ int d4_ensemble_create(void **out, int count, const int *n, const d4_params *p) 
             voff += n[k] + (n[k] & 1) + 2;  // keep every vector 16-byte aligned
             voff += voff & 1;
             moff += (long long)n[k] * n[k];
+            woff += d4::lu_mask_words_for((n[k] + d4::kLuNb - 1) / d4::kLuNb);
             smax = std::max<long long>(smax, n[k]);
         }
         E->vtot = voff;
+        E->words = woff;
+        D4_CUDA_OK(cudaDeviceGetAttribute(&E->sms, cudaDevAttrMultiProcessorCount, p->device));
         for (int v = 0; v < kNumVec; ++v) {
             D4_CUDA_OK(d4::dmalloc((void **)&E->P.v[v], sizeof(double) * voff));
             D4_CUDA_OK(cudaMemsetAsync(E->P.v[v], 0, sizeof(double) * voff, E->stream));
@@ -742,14 +614,28 @@ int d4_ensemble_create(void **out, int count, const int *n, const d4_params *p) 
         D4_CUDA_OK(d4::dmalloc((void **)&E->P.LU, sizeof(double) * moff));
         D4_CUDA_OK(cudaMemsetAsync(E->P.A, 0, sizeof(double) * moff, E->stream));
         D4_CUDA_OK(d4::dmalloc((void **)&E->P.piv, sizeof(int) * voff));
-        D4_CUDA_OK(d4::dmalloc((void **)&E->P.sing, sizeof(int) * count));
+        D4_CUDA_OK(d4::dmalloc((void **)&E->P.perm, sizeof(int) * voff));
+        D4_CUDA_OK(d4::dmalloc((void **)&E->P.lu_p0, sizeof(double) * voff * 32));
+        D4_CUDA_OK(d4::dmalloc((void **)&E->P.lu_q, sizeof(double) * voff * 64));
+        D4_CUDA_OK(d4::dmalloc((void **)&E->P.lu_u, sizeof(double) * voff * 64));
+        D4_CUDA_OK(d4::dmalloc((void **)&E->P.lu_dg, sizeof(double) * count * d4::kLuDiagWords));
+        D4_CUDA_OK(d4::dmalloc((void **)&E->P.lu_words, sizeof(unsigned) * woff));
+        D4_CUDA_OK(d4::dmalloc((void **)&E->P.lu_flags, sizeof(int) * d4::kFlagCount * count));
+        D4_CUDA_OK(d4::dmalloc((void **)&E->P.lu_maps, sizeof(d4::LuMaps) * count));
+        std::vector<d4::LuMaps> maps(count);
+        for (int k = 0; k < count; ++k) {
+            const Inst &in = E->hins[k];
+            d4::lu_encode_maps(maps[k], E->P.LU + in.moff, E->P.lu_u + in.voff * 64, in.n);
+        }
+        D4_CUDA_OK(cudaMemcpy(E->P.lu_maps, maps.data(), sizeof(d4::LuMaps) * count,
+                              cudaMemcpyHostToDevice));
         D4_CUDA_OK(d4::dmalloc((void **)&E->P.sing_any, sizeof(int) * count));
         D4_CUDA_OK(d4::dmalloc((void **)&E->P.ratio, sizeof(double) * 2 * count));
         D4_CUDA_OK(d4::dmalloc((void **)&E->P.strain, sizeof(double) * count));
         D4_CUDA_OK(cudaMemsetAsync(E->P.strain, 0, sizeof(double) * count, E->stream));
         D4_CUDA_OK(d4::dmalloc((void **)&E->P.acc, sizeof(int) * count));
-        D4_CUDA_OK(d4::dmalloc((void **)&E->P.err, sizeof(int) * 4));
-        D4_CUDA_OK(cudaMemsetAsync(E->P.err, 0, sizeof(int) * 4, E->stream));
+        D4_CUDA_OK(d4::dmalloc((void **)&E->P.err, sizeof(int) * 8));
+        D4_CUDA_OK(cudaMemsetAsync(E->P.err, 0, sizeof(int) * 8, E->stream));
         D4_CUDA_OK(d4::dmalloc((void **)&E->d_ins, sizeof(Inst) * count));
         D4_CUDA_OK(cudaMemcpyAsync(E->d_ins, E->hins.data(), sizeof(Inst) * count,
                                    cudaMemcpyHostToDevice, E->stream));
@@ -759,7 +645,10 @@ int d4_ensemble_create(void **out, int count, const int *n, const d4_params *p) 
         D4_CUDA_OK(d4::dmalloc((void **)&E->d_pre_row, sizeof(int) * (count + 1)));
         D4_CUDA_OK(d4::dmalloc((void **)&E->d_pre_mat, sizeof(int) * (count + 1)));
         E->hsc.resize(count);
-        E->solve_smem = (int)(sizeof(double) * smax);
+        E->solve_warps = (int)std::min<long long>(d4::trsv::kClusterMaxWarps, (smax + 31) / 32);
+        E->solve_smem = (int)d4::trsv::cluster_smem_bytes<double>((int)smax);
+        D4_CUDA_OK(cudaFuncSetAttribute(k_ens_lu, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)sizeof(d4::lux::Smem)));
         D4_CUDA_OK(cudaFuncSetAttribute(k_ens_solve, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         E->solve_smem));
         D4_CUDA_OK(cudaFuncSetAttribute(k_ens_rows<true>,
@@ -772,6 +661,12 @@ int d4_ensemble_create(void **out, int count, const int *n, const d4_params *p) 
     } catch (const d4::CudaError &e) {
         d4_ensemble_destroy(E);
         return D4_ERR_CUDA;
+    } catch (const d4::StateError &e) {
+        d4_ensemble_destroy(E);
+        return D4_ERR_STATE;
+    } catch (const std::bad_alloc &) {
+        d4_ensemble_destroy(E);
+        return D4_ERR_NOMEM;
     }
     *out = E;
     return D4_OK;
@@ -783,7 +678,9 @@ int d4_ensemble_destroy(void *ens) {
     if (E->stream) cudaStreamSynchronize(E->stream);
     for (int v = 0; v < d4::ens::kNumVec; ++v)
         if (E->P.v[v]) cudaFree(E->P.v[v]);
-    void *bufs[] = {E->P.F, E->P.A, E->P.LU, E->P.piv, E->P.sing, E->P.sing_any, E->P.ratio,
+    void *bufs[] = {E->P.F, E->P.A, E->P.LU, E->P.piv, E->P.perm, E->P.lu_p0, E->P.lu_q,
+                    E->P.lu_u, E->P.lu_dg, E->P.lu_words, E->P.lu_maps, E->P.lu_flags,
+                    E->P.sing_any, E->P.ratio,
                     E->P.strain,
                     E->P.acc, E->P.err, E->d_ins, E->d_sc, E->d_act, E->d_pre_pair,
                     E->d_pre_row, E->d_pre_mat};
@@ -903,11 +800,13 @@ int d4_ensemble_run(void *ens, long long max_rounds, d4_run_result *res) {
             std::vector<int> sing(E->count);
             D4_CUDA_OK(cudaMemcpyAsync(sing.data(), E->P.sing_any, sizeof(int) * E->count,
                                        cudaMemcpyDeviceToHost, E->stream));
-            int perr = 0;
-            D4_CUDA_OK(cudaMemcpyAsync(&perr, E->P.err, sizeof(int), cudaMemcpyDeviceToHost,
+            int perr[8] = {};
+            D4_CUDA_OK(cudaMemcpyAsync(perr, E->P.err, sizeof(perr), cudaMemcpyDeviceToHost,
                                        E->stream));
             D4_CUDA_OK(cudaStreamSynchronize(E->stream));
-            if (perr) throw d4::StateError("row-sum pipeline wait timed out");
+            if (perr[0]) throw d4::StateError("row-sum pipeline wait timed out");
+            if (perr[1]) throw d4::StateError("LU wait timed out");
+            if (perr[2]) throw d4::StateError("triangular solve wait timed out");
             for (int k : active) {
                 HostInst &h = E->hi[k];
                 const double hh = h.step_size;

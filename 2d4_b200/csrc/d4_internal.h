@@ -19,8 +19,8 @@ constexpr int kLuNb = 32;          // LU block width (FP64 path)
 // the FP64 form's schedule words (strip counters, look-ahead epoch); after the
 // two Q halves (2 x n x 32) the FP64 form's two U12 halves (2 x 32 x n) and the
 // published diagonal block with its reciprocals.
-constexpr int lu_pass_words(int nblk) { return nblk * 33 + 8; }
-constexpr int lu_mask_words_for(int nblk) { return lu_pass_words(nblk) + nblk + 64; }
+__host__ __device__ constexpr int lu_pass_words(int nblk) { return nblk * 33 + 8; }
+__host__ __device__ constexpr int lu_mask_words_for(int nblk) { return lu_pass_words(nblk) + nblk + 64; }
 constexpr int kLuDiagWords = kLuNb * (kLuNb + 1) + kLuNb;
 constexpr int kSolveThreads = 1024;
 constexpr int kMaxSolveN = 8192;   // x and g of the one-CTA solve live in shared memory

@@ -1,6 +1,6 @@
 // d4_lu_exact.cuh: FP64 LU with exact partial pivoting in the oracle's
-// operation order, by a group of CTAs (the grid of a cooperative launch).
-// Compiled with --fmad=false.
+// operation order, by a group of CTAs (the grid of a cooperative launch, or one
+// thread-block cluster).  Compiled with --fmad=false.
 //
 // Same result, bit for bit, as the oracle's right-looking Gaussian elimination
 // with partial pivoting (first index of the largest |a_ik| wins; an exact zero
@@ -219,6 +219,35 @@ struct GridGroup {
     }
 };
 
+// One thread-block cluster (all its CTAs run together by construction).
+struct ClusterGroup {
+    __device__ int rank() const {
+        unsigned r;
+        asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+        return (int)r;
+    }
+    __device__ int size() const {
+        unsigned r;
+        asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+        return (int)r;
+    }
+    __device__ void arrive(bool) {
+        fence_bulk();
+        __syncthreads();
+        arrive_quiet(false);
+    }
+    __device__ void arrive_quiet(bool) {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    }
+    __device__ unsigned wait(const unsigned *mask, int *) {
+        Smem &S = smem();
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (threadIdx.x == 0) S.verdict = mask ? ld_acq(mask) : 0u;
+        __syncthreads();
+        return S.verdict;
+    }
+};
+
 // Source row in P0 of position r after the block's transpositions (applied in
 // order to the arrangement): walk the list backwards.
 __device__ __forceinline__ int src_row(int r, const int *sa, const int *sb, int ns) {
@@ -363,7 +392,7 @@ __device__ __forceinline__ unsigned eliminate(double (&c)[4], bool &bad) {
 // The same elimination with IEEE divisions, for blocks with values outside the
 // quotient window or zero pivots, and for passes that skip singular columns.
 // All threads call it (warps 0..7 pass their columns, the others idle).
-__device__ __noinline__ unsigned eliminate_slow(const double (&c0)[4], int kw,
+static __device__ __noinline__ unsigned eliminate_slow(const double (&c0)[4], int kw,
                                                 unsigned skip) {
     Smem &S = smem();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -405,7 +434,7 @@ __device__ __noinline__ unsigned eliminate_slow(const double (&c0)[4], int kw,
 
 // Eliminates c by the fast path, or the slow one where that has to be; all
 // threads call it.  Afterwards S.s, S.q and S.rs are complete.
-__device__ __noinline__ unsigned eliminate_any(const double (&c0)[4], int kw,
+static __device__ __noinline__ unsigned eliminate_any(const double (&c0)[4], int kw,
                                                   unsigned skip) {
     Smem &S = smem();
     unsigned msk = 0;
@@ -423,7 +452,7 @@ __device__ __noinline__ unsigned eliminate_any(const double (&c0)[4], int kw,
 
 // The diagonal block of a pass from P0 (block 0, and passes after a swap), in
 // every CTA; CTA 0 stores the pre-division values.  All threads call it.
-__device__ __noinline__ unsigned diag_from_p0(const Args &a, double *Q, int k0, int kw,
+static __device__ __noinline__ unsigned diag_from_p0(const Args &a, double *Q, int k0, int kw,
                                               int ns, unsigned skip, bool write_q) {
     Smem &S = smem();
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
@@ -468,7 +497,7 @@ __device__ __forceinline__ void row_store(const Args &a, double *Q, int r_pos, i
 
 // A row with IEEE divisions, for values outside the quotient window and passes
 // that skip singular columns.  Returns the row's flags.
-__device__ __noinline__ unsigned row_below_slow(const Args &a, double *Q, int r_pos, int sr, int k0,
+static __device__ __noinline__ unsigned row_below_slow(const Args &a, double *Q, int r_pos, int sr, int k0,
                                                 unsigned skip, bool active) {
     Smem &S = smem();
     const int lane = threadIdx.x & 31, q = lane % kLanes, gb = lane - q;
@@ -646,7 +675,7 @@ __device__ __forceinline__ void publish(const Args &a, const double (&c)[4], int
 
 // The look-ahead after a pass that needed a swap (or by a single CTA): L21 and
 // U12 as the pass left them.
-__device__ __noinline__ void look_ahead(const Args &a, int k0, int kb, int pass,
+static __device__ __noinline__ void look_ahead(const Args &a, int k0, int kb, int pass,
                                         const double *U) {
     Smem &S = smem();
     const int n = a.n, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
@@ -682,7 +711,7 @@ __device__ __noinline__ void look_ahead(const Args &a, int k0, int kb, int pass,
 // first row also store U12 to A; tiles of the first column hold the next
 // block's columns, whose new values go to P0 instead of A.
 template <int RM, int RN>
-__device__ __noinline__ unsigned update_tiles(const Args &a, int k0, int kb, const double *U,
+static __device__ __noinline__ unsigned update_tiles(const Args &a, int k0, int kb, const double *U,
                                               int ntr, int ntc, int first, int stride, int end,
                                               unsigned seq) {
     Smem &S = smem();

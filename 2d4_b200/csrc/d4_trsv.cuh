@@ -163,10 +163,10 @@ __device__ __forceinline__ void tile_async(const T *__restrict__ LU, int n, int 
 // A^T x = g (P A = L U, so A^T = U^T L^T P): the forward pass is U^T (lower,
 // divided), the backward pass L^T (unit upper), g is taken unpermuted and the
 // result scattered through perm at the end.
-template <bool kFwd, typename T, bool kTrans = false>
-__global__ void __launch_bounds__(32 * kClusterMaxWarps) k_trsv_cluster(
-    int n, const T *__restrict__ LU, const int *__restrict__ perm, const int *__restrict__ flags,
-    GArgs ga, T *xg, const T *xin, int *err) {
+template <bool kFwd, typename T, bool kTrans>
+__device__ __forceinline__ void solve_pass(int n, const T *__restrict__ LU,
+                                           const int *__restrict__ perm, const int *flags,
+                                           const GArgs &ga, T *xg, const T *xin, int *err) {
     extern __shared__ __align__(16) unsigned char craw[];
     const int nblk = (n + 31) / 32;
     T *xall = reinterpret_cast<T *>(craw);
@@ -331,6 +331,25 @@ __global__ void __launch_bounds__(32 * kClusterMaxWarps) k_trsv_cluster(
     }
     __syncthreads();
     cluster_sync_all();
+}
+
+// Between two passes of one launch by a lone CTA: frees the first pass's
+// barriers, so that the second can set them up again.
+__device__ __forceinline__ void release_barriers(int n, size_t elem) {
+    extern __shared__ __align__(16) unsigned char craw[];
+    uint64_t *mbar = reinterpret_cast<uint64_t *>(craw + ((elem * (size_t)n + 15) / 16) * 16);
+    for (int b = threadIdx.x; b < 4 * ((n + 31) / 32); b += blockDim.x)
+        asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(
+                         static_cast<uint32_t>(__cvta_generic_to_shared(mbar + b)))
+                     : "memory");
+    __syncthreads();
+}
+
+template <bool kFwd, typename T, bool kTrans = false>
+__global__ void __launch_bounds__(32 * kClusterMaxWarps) k_trsv_cluster(
+    int n, const T *__restrict__ LU, const int *__restrict__ perm, const int *__restrict__ flags,
+    GArgs ga, T *xg, const T *xin, int *err) {
+    solve_pass<kFwd, T, kTrans>(n, LU, perm, flags, ga, xg, xin, err);
 }
 
 // Forward then backward cluster solve on `stream`: x1 = forward result (global
