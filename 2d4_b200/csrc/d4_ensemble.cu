@@ -96,7 +96,7 @@ __device__ __forceinline__ int find_slot(const int *pre, int na, int b) {
 }
 
 template <bool kJac>
-__global__ void __launch_bounds__(256) k_ens_pairs(Pools P, const Inst *ins, const Sc *sc,
+__global__ void __launch_bounds__(256, pair_min_blocks(kJac, false)) k_ens_pairs(Pools P, const Inst *ins, const Sc *sc,
                                                    const int *act, const int *pre, int na,
                                                    Common cm, int xsel, double hmul) {
     const int s = find_slot(pre, na, blockIdx.x);
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(256) k_ens_pairs(Pools P, const Inst *ins, con
 }
 
 template <bool kJac>
-__global__ void __launch_bounds__(64) k_ens_rows(Pools P, const Inst *ins, const Sc *sc,
+__global__ void __launch_bounds__(kRowThreads) k_ens_rows(Pools P, const Inst *ins, const Sc *sc,
                                                  const int *act, const int *pre, int na,
                                                  Common cm, int ea, int eb, int va, int vb) {
     const int s = find_slot(pre, na, blockIdx.x);
@@ -394,7 +394,7 @@ void sweep(Ensemble &E, int xsel, double hmul, int ea, int eb, int va, int vb) {
         E.P, E.d_ins, E.d_sc, E.d_act, E.d_pre_pair, na, E.cm, xsel, hmul);
     check("k_ens_pairs");
     constexpr int bytes = row_smem_bytes<kJac>();
-    k_ens_rows<kJac><<<E.pre_row[na], 64, bytes, E.stream>>>(
+    k_ens_rows<kJac><<<E.pre_row[na], kRowThreads, bytes, E.stream>>>(
         E.P, E.d_ins, E.d_sc, E.d_act, E.d_pre_row, na, E.cm, ea, eb, va, vb);
     check("k_ens_rows");
     if (kJac) {
@@ -405,8 +405,8 @@ void sweep(Ensemble &E, int xsel, double hmul, int ea, int eb, int va, int vb) {
 }
 
 // Pair-tile autotuner of the ensemble: threads per tile from the candidates,
-// by timing the stress and fused pair kernels of every active instance
-// (tolerances off; F and A are scratch that every attempt rewrites), one
+// by timing the stress and fused pair kernels on the active instances' first
+// kTuneTiles tiles (tolerances off; F and A are scratch that every attempt rewrites), one
 // untimed and three timed runs each; the fastest total wins.  Each pair is
 // evaluated by one thread whatever the choice, so results do not depend on it.
 void autotune(Ensemble &E) {
@@ -414,6 +414,7 @@ void autotune(Ensemble &E) {
     Common cm = E.cm;
     cm.use_dipole = 0;
     const int na = (int)E.act.size();
+    const int tiles = std::min(E.pre_pair[na], kTuneTiles);
     float best = 1e30f;
     int best_ty = 8;
     cudaEvent_t e0, e1;  // own events: E.ev0 times the whole d4_ensemble_run call
@@ -423,9 +424,9 @@ void autotune(Ensemble &E) {
         float total = 0;
         for (int rep = 0; rep < 4; ++rep) {
             D4_CUDA_OK(cudaEventRecord(e0, E.stream));
-            k_ens_pairs<false><<<E.pre_pair[na], dim3(kTile, ty), 0, E.stream>>>(
+            k_ens_pairs<false><<<tiles, dim3(kTile, ty), 0, E.stream>>>(
                 E.P, E.d_ins, E.d_sc, E.d_act, E.d_pre_pair, na, cm, kX0, 1.0);
-            k_ens_pairs<true><<<E.pre_pair[na], dim3(kTile, ty), 0, E.stream>>>(
+            k_ens_pairs<true><<<tiles, dim3(kTile, ty), 0, E.stream>>>(
                 E.P, E.d_ins, E.d_sc, E.d_act, E.d_pre_pair, na, cm, kX0, 1.0);
             check("k_ens_pairs<tune>");
             D4_CUDA_OK(cudaEventRecord(e1, E.stream));

@@ -33,7 +33,7 @@ struct Hyp {
     double ch0, sh0, chp1, chm1, shp1, shm1, chp2, chm2, shp2, shm2;
     double chp3, chm3, chp4, chm4, chp5, chm5;
     __device__ __forceinline__ explicit Hyp(double e) {
-        const double inv = 1 / e;
+        const double inv = f64::recip(e);
         const double s = (e + inv) * 0.5, d = (e - inv) * 0.5;
         ch0 = s;
         sh0 = d;
@@ -54,54 +54,51 @@ struct Hyp {
     }
 };
 
-// One image: f_l and, when wanted, f_dx_l (sh = ch for |i| >= 3), from r = 1/q.
-__device__ __forceinline__ double f_l(double dx, double c, double ch) {
-    const double r = 1 / (ch - c);
-    return (2 * kPi * kPi) * dx * (ch * c - 1) * (r * r);
+// One image: f_l and, with kGrad, f_dx_l (sh = ch for |i| >= 3), from r = 1/q
+// (within an ulp: Newton steps from the hardware's estimate).
+template <bool kGrad>
+__device__ __forceinline__ void image(double u, double c, double ch, double sh, double &f,
+                                      double &g) {
+    const double r = f64::recip(ch - c);
+    const double n1 = ch * c - 1, w = n1 * (r * r);
+    f = k2Pi2 * u * w;
+    if (kGrad) g = (w + (2 * kPi) * u * (sh * c * (r * r) - 2 * sh * (w * r))) * k2Pi2;
 }
 
-__device__ __forceinline__ double f_dx_l(double dx, double c, double ch, double sh) {
-    const double r = 1 / (ch - c);
-    const double r2 = r * r;
-    const double n1 = ch * c - 1;
-    return (n1 * r2 + (2 * kPi) * dx * (sh * c * r2 - 2 * n1 * sh * (r2 * r))) * k2Pi2;
-}
-
-__device__ __forceinline__ double f_0(double dx, double c, double dy, double ch) {
-    if (dx * dx + dy * dy > 1e-6) return f_l(dx, c, ch);
-    return f64::f_0(dx, c, dy, ch);
-}
-
-__device__ __forceinline__ double f_dx_0(double dx, double c, double dy, double ch, double sh) {
-    if (dx * dx + dy * dy > 1e-6) return f_dx_l(dx, c, ch, sh);
-    return f64::f_dx_0(dx, c, dy, ch, sh);
-}
-
-// Field::xy and Field::xy_diff_x (4-arg) over the same images and blends as
-// d4::f64::xy / xy_diff_x.
-__device__ __forceinline__ double xy(double dx, double dy, const Hyp &h, double c) {
-    const double g3 = f_l(dx + 3, c, h.chp3) + f_l(dx - 3, c, h.chm3) + f_l(dx + 2, c, h.chp2) +
-                      f_l(dx - 2, c, h.chm2) + f_l(dx + 1, c, h.chp1) + f_l(dx - 1, c, h.chm1) +
-                      f_0(dx, c, dy, h.ch0);
-    if (dx < 0)
-        return f_l(dx + 5, c, h.chp5) * (0 - dx) + f_l(dx - 4, c, h.chm4) * (1 + dx) +
-               f_l(dx + 4, c, h.chp4) + g3;
-    return f_l(dx - 5, c, h.chm5) * dx + f_l(dx + 4, c, h.chp4) * (1 - dx) +
-           f_l(dx - 4, c, h.chm4) + g3;
-}
-
-__device__ __forceinline__ double xy_diff_x(double dx, double dy, const Hyp &h, double c) {
-    const double g3 = f_dx_0(dx, c, dy, h.ch0, h.sh0) + f_dx_l(dx + 1, c, h.chp1, h.shp1) +
-                      f_dx_l(dx - 1, c, h.chm1, h.shm1) + f_dx_l(dx + 2, c, h.chp2, h.shp2) +
-                      f_dx_l(dx - 2, c, h.chm2, h.shm2) + f_dx_l(dx + 3, c, h.chp3, h.chp3) +
-                      f_dx_l(dx - 3, c, h.chm3, h.chm3);
-    if (dx < 0)
-        return f_dx_l(dx + 5, c, h.chp5, h.chp5) * (0 - dx) - f_l(dx + 5, c, h.chp5) +
-               f_dx_l(dx - 4, c, h.chm4, h.chm4) * (1 + dx) + f_l(dx - 4, c, h.chm4) +
-               f_dx_l(dx + 4, c, h.chp4, h.chp4) + g3;
-    return f_dx_l(dx - 5, c, h.chm5, h.chm5) * dx + f_l(dx - 5, c, h.chm5) +
-           f_dx_l(dx + 4, c, h.chp4, h.chp4) * (1 - dx) - f_l(dx + 4, c, h.chp4) +
-           f_dx_l(dx - 4, c, h.chm4, h.chm4) + g3;
+// Field::xy and, with kGrad, Field::xy_diff_x over the same images and blends as
+// d4::f64::pair.
+template <bool kGrad>
+__device__ __forceinline__ void pair(double dx, double dy, double &f, double &g) {
+    const double c = cos2piy(dy);
+    const Hyp h(exp2pix(dx));
+    double t, u;
+    image<kGrad>(dx + 3, c, h.chp3, h.chp3, f, g);
+    auto add = [&](double v, double ch, double sh) {
+        image<kGrad>(v, c, ch, sh, t, u);
+        f += t;
+        if (kGrad) g += u;
+    };
+    add(dx - 3, h.chm3, h.chm3);
+    add(dx + 2, h.chp2, h.shp2);
+    add(dx - 2, h.chm2, h.shm2);
+    add(dx + 1, h.chp1, h.shp1);
+    add(dx - 1, h.chm1, h.shm1);
+    if (dx * dx + dy * dy > 1e-6) {
+        add(dx, h.ch0, h.sh0);
+    } else {
+        f += f64::f_0(dx, c, dy, h.ch0);
+        if (kGrad) g += f64::f_dx_0(dx, c, dy, h.ch0, h.sh0);
+    }
+    const bool neg = dx < 0;
+    const double far = fabs(dx), sg = neg ? -1.0 : 1.0;
+    const double ch5 = neg ? h.chp5 : h.chm5, ch4b = neg ? h.chm4 : h.chp4;
+    add(dx - 4 * sg, neg ? h.chp4 : h.chm4, neg ? h.chp4 : h.chm4);
+    image<kGrad>(dx - 5 * sg, c, ch5, ch5, t, u);
+    f += t * far;
+    if (kGrad) g += u * far + t * sg;
+    image<kGrad>(dx + 4 * sg, c, ch4b, ch4b, t, u);
+    f += t * (1 - far);
+    if (kGrad) g += u * (1 - far) - t * sg;
 }
 
 }  // namespace f64fast

@@ -1,6 +1,7 @@
 // d4_fp64.cu: FP64 pair sweeps and small kernels of the plain form (compiled
 // with --fmad=false).  The pair tiles and the ordered row sums live in
 // d4_sweep64.cuh.
+#include <algorithm>
 #include <cstdint>
 #include <map>
 #include <mutex>
@@ -118,7 +119,7 @@ static void launch_rows(Ctx &c, const RowArgs &r, cudaStream_t st) {
     constexpr int bytes = row_smem_bytes<kJac>();
     D4_CUDA_OK(cudaFuncSetAttribute(k_rows64<kJac>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     bytes));
-    k_rows64<kJac><<<(c.n + kRowRows - 1) / kRowRows, 64, bytes, st>>>(r);
+    k_rows64<kJac><<<(c.n + kRowRows - 1) / kRowRows, kRowThreads, bytes, st>>>(r);
     check_launch(kJac ? "k_rows64<jacobian>" : "k_rows64<speeds>");
 }
 
@@ -213,6 +214,7 @@ void autotune_pairs(Ctx &c) {
     a.F = c.F;
     a.A = c.A;
     a.h = c.step_size;
+    const int tiles = std::min(pair_blocks(c.n), kTuneTiles);
     float best = 1e30f;
     int best_ty = 8;
     for (int ty : kPairTyCandidates) {
@@ -220,11 +222,11 @@ void autotune_pairs(Ctx &c) {
         for (int rep = 0; rep < 4; ++rep) {
             D4_CUDA_OK(cudaEventRecord(c.ev0, c.stream));
             if (c.tab) {
-                k_pairs64<false, true><<<pair_blocks(c.n), dim3(kTile, ty), 0, c.stream>>>(a);
-                k_pairs64<true, true><<<pair_blocks(c.n), dim3(kTile, ty), 0, c.stream>>>(a);
+                k_pairs64<false, true><<<tiles, dim3(kTile, ty), 0, c.stream>>>(a);
+                k_pairs64<true, true><<<tiles, dim3(kTile, ty), 0, c.stream>>>(a);
             } else {
-                k_pairs64<false><<<pair_blocks(c.n), dim3(kTile, ty), 0, c.stream>>>(a);
-                k_pairs64<true><<<pair_blocks(c.n), dim3(kTile, ty), 0, c.stream>>>(a);
+                k_pairs64<false><<<tiles, dim3(kTile, ty), 0, c.stream>>>(a);
+                k_pairs64<true><<<tiles, dim3(kTile, ty), 0, c.stream>>>(a);
             }
             check_launch("k_pairs64<tune>");
             D4_CUDA_OK(cudaEventRecord(c.ev1, c.stream));

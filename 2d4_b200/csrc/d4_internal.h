@@ -289,6 +289,9 @@ void field_eval64(Ctx &c, int count, const double *dx, const double *dy, double 
 void autotune_pairs(Ctx &c);
 // The candidates and the timing shared with the ensemble's tuner.
 constexpr int kPairTyCandidates[3] = {2, 4, 8};
+// Tiles timed: several waves of blocks, so the choice is the whole sweep's (an
+// ensemble of 192 instances has 141,000 tiles, whose tuning took 96 ms).
+constexpr int kTuneTiles = 8192;
 
 // ---- FP64 factorisation and solves (d4_lu64.cu) ----
 // Factorises A into LU; returns via flags whether the pivoted path ran and

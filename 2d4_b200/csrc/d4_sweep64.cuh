@@ -45,15 +45,15 @@ __device__ __forceinline__ void tol_min(double *tol, int idx, double d) {
 
 // Enumerates upper-triangular tiles (ti <= tj) from a linear block index.
 __device__ __forceinline__ void tile_of(int t, int T, int &ti, int &tj) {
-    // row ti holds T - ti tiles; walk rows (T is small: <= 256 for n <= 8192)
-    int r = 0;
-    int rem = t;
-    while (rem >= T - r) {
-        rem -= T - r;
-        ++r;
-    }
+    // row r starts at r T - r (r - 1) / 2: the quadratic's root in FP32, then the
+    // exact row (T <= 256, so the estimate is off by one at most)
+    const float b = (float)(2 * T + 1);
+    int r = (int)((b - sqrtf(b * b - 8.0f * (float)t)) * 0.5f);
+    r = max(0, min(r, T - 1));
+    while (r > 0 && r * T - r * (r - 1) / 2 > t) --r;
+    while (r < T - 1 && (r + 1) * T - (r + 1) * r / 2 <= t) ++r;
     ti = r;
-    tj = r + rem;
+    tj = r + t - (r * T - r * (r - 1) / 2);
 }
 
 struct PairArgs {
@@ -92,6 +92,12 @@ inline PairArgs pair_args(const Ctx &c, const double *x, const double *y) {
     return a;
 }
 
+// Blocks of 256 threads per SM that the registers are bounded for.  The fused
+// tiles at N=2000: 303 us unbounded (152 registers, one block) and with a
+// division per quotient, 94, 91 and 91 us with 2, 3 and 4 blocks; the mixed
+// form's at N=4096 568, then 252, 222 and 235 us; the table's 35, 45, 36 us.
+constexpr int pair_min_blocks(bool jac, bool table) { return jac && !table ? 3 : 4; }
+
 inline int pair_blocks(int n) {
     const int T = (n + kTile - 1) / kTile;
     return T * (T + 1) / 2;
@@ -124,10 +130,13 @@ __device__ __forceinline__ void pair_tile(const PairArgs &a, int tile) {
     for (int lj = ty; lj < kTile; lj += blockDim.y) {
         const int j = j0 + lj;
         double f = 0, v = 0;
-        if (i < a.n && j < a.n && i < j) {
-            double dx = D4_PAIR_FIELD::normalize(sxi[tx] - sxj[lj]);
-            double dy = D4_PAIR_FIELD::normalize(syi[tx] - syj[lj]);
-            double dist_sq = dx * dx + dy * dy;
+        const bool valid = i < a.n && j < a.n && i < j;
+        const double dx = D4_PAIR_FIELD::normalize(sxi[tx] - sxj[lj]);
+        const double dy = D4_PAIR_FIELD::normalize(syi[tx] - syj[lj]);
+        const double dist_sq = dx * dx + dy * dy;
+        // a warp with no pair inside the Jacobian's range skips the derivative
+        const bool grad = kJac && __any_sync(0xffffffffu, valid && dist_sq < a.range_sq * a.cut_sq);
+        if (valid) {
             if (a.tol && dist_sq < a.min_prec_sq) {
                 row_min = fmin(row_min, dist_sq);
                 tol_min(a.tol, j, dist_sq);
@@ -138,12 +147,10 @@ __device__ __forceinline__ void pair_tile(const PairArgs &a, int tile) {
                 const double2 t = tab::eval<kJac>(a.tb, dx, dy);
                 fxy = t.x;
                 fdx = t.y;
+            } else if (grad) {
+                D4_PAIR_FIELD::pair<true>(dx, dy, fxy, fdx);
             } else {
-                D4_PAIR_FIELD::Hyp hp(D4_PAIR_FIELD::exp2pix(dx));
-                double c = D4_PAIR_FIELD::cos2piy(dy);
-                fxy = D4_PAIR_FIELD::xy(dx, dy, hp, c);
-                if (kJac && dist_sq < a.range_sq * a.cut_sq)
-                    fdx = D4_PAIR_FIELD::xy_diff_x(dx, dy, hp, c);
+                D4_PAIR_FIELD::pair<false>(dx, dy, fxy, fdx);
             }
             f = fxy * bi * bj;
             if (kJac) {
@@ -175,21 +182,27 @@ __device__ __forceinline__ void pair_tile(const PairArgs &a, int tile) {
 }
 
 template <bool kJac, bool kTab = false>
-__global__ void __launch_bounds__(256) k_pairs64(PairArgs a) {
+__global__ void __launch_bounds__(256, pair_min_blocks(kJac, kTab)) k_pairs64(PairArgs a) {
     pair_tile<kJac, kTab>(a, blockIdx.x);
 }
 
 // Ordered row sums, pipelined.  Block b owns rows i0 = 32 b .. i0 + 31; F (and,
 // in the fused sweep, the raw Jacobian A) are column-major, so the 32 rows of
-// one column are 256 contiguous bytes.  Warp 1 streams them column chunk by
-// column chunk into shared memory with bulk copies (kRowStages chunks of
-// kRowCols columns in flight, each completing on its stage's mbarrier); warp 0
-// has one lane per row and adds the entries in ascending j, exactly the
-// reference's summation order (src/simulation.cpp:292-311,444-503).  The fused
-// sweep then writes subSum, d_i = weight(subSum) and the row scale (1 + d_i)/2
-// for k_scale_rows64.  A wait that gives up records err[0] = 1 and the block
-// drains its copies in flight before it returns.
-constexpr int kRowRows = 32, kRowCols = 64, kRowStages = 4;
+// one column are 256 contiguous bytes.  Warps 1..kRowProducers copy them chunk
+// by chunk into shared memory (16-byte cp.async, kRowStages chunks of kRowCols
+// columns in flight, each completing on its stage's mbarrier); warp 0 has one
+// lane per row and adds the entries in ascending j, exactly the reference's
+// summation order (src/simulation.cpp:292-311,444-503).  Its loop reads eight
+// columns ahead of the dependent additions, and only the chunk that holds the
+// rows' own columns tests for them.  The chain of n additions (8.5 cycles each)
+// and the memory's bandwidth bound it; a bulk copy per column (about 65 cycles
+// of issue each) and a test per column took 60 cycles a column, 112 fused
+// (N=4096: 130 and 247 us).  The fused sweep then writes subSum, d_i =
+// weight(subSum) and the row scale (1 + d_i)/2 for k_scale_rows64.  A wait that
+// gives up records err[0] = 1; the producers wait for their own copies before
+// the block returns.
+constexpr int kRowRows = 32, kRowCols = 64, kRowStages = 4, kRowProducers = 4;
+constexpr int kRowThreads = 32 * (1 + kRowProducers);
 
 struct RowArgs {
     int n;
@@ -206,13 +219,17 @@ constexpr int row_smem_bytes() {
     return (kJac ? 2 : 1) * kRowStages * kRowCols * kRowRows * (int)sizeof(double);
 }
 
+__device__ __forceinline__ void row_copy16(double *dst, const double *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(bulk::smem_u32(dst)), "l"(src)
+                 : "memory");
+}
+
 template <bool kJac>
 __device__ __forceinline__ void row_block(const RowArgs &a, int rb) {
     extern __shared__ __align__(128) unsigned char row_smem[];
     double *bf = reinterpret_cast<double *>(row_smem);  // [stage][col][row]
     double *ba = bf + kRowStages * kRowCols * kRowRows;
     __shared__ __align__(8) uint64_t full[kRowStages], empty[kRowStages];
-    __shared__ int issued_s, consumed_s;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n = a.n;
     const int i0 = rb * kRowRows;
@@ -220,36 +237,35 @@ __device__ __forceinline__ void row_block(const RowArgs &a, int rb) {
     const int nst = (n + kRowCols - 1) / kRowCols;
     if (threadIdx.x == 0) {
         for (int s = 0; s < kRowStages; ++s) {
-            bulk::init(&full[s], 1);
+            bulk::init(&full[s], 32 * kRowProducers);
             bulk::init(&empty[s], 1);
         }
         bulk::fence_init();
-        issued_s = 0;
-        consumed_s = 0;
     }
     __syncthreads();
-    if (warp == 1) {
-        // producer
-        const uint32_t col_bytes = rows * (uint32_t)sizeof(double);
-        int st = 0;
-        for (; st < nst; ++st) {
+    if (warp > 0) {
+        // producers: thread -> row pair and every (2 kRowProducers)-th column
+        const int t = threadIdx.x - 32, r = 2 * (t & 15), c0 = t >> 4;
+        const double *pf = a.F + i0 + r, *pa = a.A + i0 + r;
+        for (int st = 0; st < nst; ++st) {
             const int s = st % kRowStages;
             const uint32_t use = st / kRowStages;
-            if (use > 0 && !__all_sync(0xffffffffu, bulk::wait(&empty[s], (use - 1) & 1))) {
-                if (lane == 0) atomicOr(a.err, 1);
+            if (use > 0 && !bulk::wait(&empty[s], (use - 1) & 1)) {
+                atomicOr(a.err, 1);
                 break;
             }
             const int j0 = st * kRowCols, nc = min(kRowCols, n - j0);
-            if (lane == 0) bulk::arrive_expect_tx(&full[s], nc * col_bytes * (kJac ? 2 : 1));
-            __syncwarp();
-            for (int k = lane; k < nc; k += 32) {
-                const size_t off = (size_t)i0 + (size_t)(j0 + k) * n;
-                const int slot = (s * kRowCols + k) * kRowRows;
-                bulk::g2s(bf + slot, a.F + off, col_bytes, &full[s]);
-                if (kJac) bulk::g2s(ba + slot, a.A + off, col_bytes, &full[s]);
-            }
+            if (r < rows)  // n is even: pairs never straddle the edge
+                for (int c = c0; c < nc; c += 2 * kRowProducers) {
+                    const int slot = (s * kRowCols + c) * kRowRows + r;
+                    row_copy16(bf + slot, pf + (size_t)(j0 + c) * n);
+                    if (kJac) row_copy16(ba + slot, pa + (size_t)(j0 + c) * n);
+                }
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(
+                             bulk::smem_u32(&full[s]))
+                         : "memory");
         }
-        if (lane == 0) issued_s = st;
+        asm volatile("cp.async.wait_all;" ::: "memory");
     } else {
         // consumer: lane = row
         const int i = i0 + lane;
@@ -264,15 +280,31 @@ __device__ __forceinline__ void row_block(const RowArgs &a, int rb) {
             const int j0 = st * kRowCols, nc = min(kRowCols, n - j0);
             const double *cf = bf + s * kRowCols * kRowRows + lane;
             const double *ca = ba + s * kRowCols * kRowRows + lane;
-            for (int k = 0; k < nc; ++k) {
-                if (j0 + k == i) continue;
-                sum += cf[k * kRowRows];
-                if (kJac) sub -= ca[k * kRowRows];
+            if (nc == kRowCols && (i0 + kRowRows <= j0 || i0 >= j0 + kRowCols)) {
+#pragma unroll 2
+                for (int k = 0; k < kRowCols; k += 8) {
+                    double f[8], g[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        f[e] = cf[(k + e) * kRowRows];
+                        if (kJac) g[e] = ca[(k + e) * kRowRows];
+                    }
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        sum += f[e];
+                        if (kJac) sub -= g[e];
+                    }
+                }
+            } else {
+                for (int k = 0; k < nc; ++k) {
+                    if (j0 + k == i) continue;
+                    sum += cf[k * kRowRows];
+                    if (kJac) sub -= ca[k * kRowRows];
+                }
             }
             __syncwarp();
             if (lane == 0) bulk::arrive(&empty[s]);
         }
-        if (lane == 0) consumed_s = st;
         if (st == nst && lane < rows) {
             const double b = bsign(i, n);
             if (kJac) {
@@ -287,15 +319,10 @@ __device__ __forceinline__ void row_block(const RowArgs &a, int rb) {
             }
         }
     }
-    __syncthreads();
-    // after a failed wait: let the copies in flight land before the block exits
-    if (threadIdx.x == 32)
-        for (int st = consumed_s; st < issued_s; ++st)
-            bulk::wait(&full[st % kRowStages], (st / kRowStages) & 1);
 }
 
 template <bool kJac>
-__global__ void __launch_bounds__(64) k_rows64(RowArgs a) {
+__global__ void __launch_bounds__(kRowThreads) k_rows64(RowArgs a) {
     row_block<kJac>(a, blockIdx.x);
 }
 
