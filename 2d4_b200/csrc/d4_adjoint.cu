@@ -50,7 +50,11 @@ inline int nb(long long n, int t) { return (int)((n + t - 1) / t); }
 //   d g_i = sum_j b_i b_j tt_ij (dz_i - dz_j),
 //   (dJt[dz] w)_i = sum_j b_i b_j tt_ij (dz_i - dz_j)(w_i - w_j).
 enum { kModeJv = 0, kModeJt = 1, kModeJvp = 2, kModeVjp = 3 };
-constexpr int kPT = 128;
+constexpr int kPT = 128;  // rows per block, one per thread
+// Columns per block: enough blocks for the chip at every n (128-column blocks
+// left N=1024 with 64 of them, 0.37-1.18 ms a sweep), fewer partial sums at
+// large n.
+__host__ __device__ constexpr int cols_per_block(int n) { return n <= 2048 ? 16 : 64; }
 
 struct DerivArgs {
     int n;
@@ -67,13 +71,21 @@ struct DerivArgs {
 //           o3 = sum bb tt (a_i - a_j)(r_i - r_j), o4 = Jt q, o5 = Jt r
 // kModeVjp: o0 = sum bb [sp (a_i - a_j) + tt ((p_i - p_j)(q_i - q_j)
 //                         + (r_i - r_j)(s_i - s_j) + (u_i + u_j))]
-// Grid: (row tiles, column tiles) of kPT x kPT pairs; block (bx, by) sums the
-// pairs of its rows with the columns of tile by and writes the partial sums to
-// part[(out * tiles + by) * n + i]; k_deriv_sum then adds the tiles in order
+// Grid: (row tiles, column tiles) of kPT x cols_per_block pairs; block (bx, by)
+// sums the pairs of its rows with the columns of tile by and writes the partial sums to
+// part[(out * tiles + by) * n + i]; k_deriv_sum then adds the tiles in a fixed order
 // (deterministic results).
+//
+// Bound by the FP64 arithmetic of the images and, at small n, by the blocks in
+// flight: 16-column blocks give N=1024 512 of them (64 before), each image takes
+// one reciprocal for its quotients, and the two second-order terms of a pair share
+// the exponential and the cosine (N=1024: Vjp 1182 -> 94 us, Jt 511 -> 50, Jv
+// 367 -> 42; the sum of the tiles 23 -> 4 us with 8 warps per 32 rows).
 template <int kMode>
 __global__ void __launch_bounds__(kPT) k_deriv(DerivArgs A, double *part) {
-    __shared__ double sx[kPT], sy[kPT], s1[kPT], s2[kPT], s3[kPT], s4[kPT], s5[kPT], s6[kPT];
+    constexpr int kMaxCols = 64;
+    __shared__ double sx[kMaxCols], sy[kMaxCols], s1[kMaxCols], s2[kMaxCols], s3[kMaxCols],
+        s4[kMaxCols], s5[kMaxCols], s6[kMaxCols];
     const int n = A.n;
     const int i = blockIdx.x * kPT + threadIdx.x;
     const bool own = i < n;
@@ -96,9 +108,9 @@ __global__ void __launch_bounds__(kPT) k_deriv(DerivArgs A, double *part) {
     }
     double o[6] = {0, 0, 0, 0, 0, 0};
     {
-        const int j0 = blockIdx.y * kPT;
+        const int cols = cols_per_block(n), j0 = blockIdx.y * cols;
         const int j = j0 + threadIdx.x;
-        if (j < n) {
+        if ((int)threadIdx.x < cols && j < n) {
             sx[threadIdx.x] = A.x[j];
             sy[threadIdx.x] = A.y[j];
             s1[threadIdx.x] = A.a ? A.a[j] : 0;
@@ -116,7 +128,7 @@ __global__ void __launch_bounds__(kPT) k_deriv(DerivArgs A, double *part) {
             }
         }
         __syncthreads();
-        const int jn = own ? min(kPT, n - j0) : 0;
+        const int jn = own ? min(cols, n - j0) : 0;
         for (int t = 0; t < jn; ++t) {
             const int jj = j0 + t;
             if (jj == i) continue;
@@ -132,15 +144,18 @@ __global__ void __launch_bounds__(kPT) k_deriv(DerivArgs A, double *part) {
                 o[0] += sp * (ai - s1[t]);
                 o[1] += sp * (ci - s2[t]);
             } else if (kMode == kModeJt) {
-                const f64::Hyp h(f64::exp2pix(dxo));
-                const double st = f64::xy_diff_x(dxo, dyo, h, f64::cos2piy(dyo)) * bb;
+                double fxy, fdx;
+                f64::pair<true>(dxo, dyo, fxy, fdx);
+                const double st = fdx * bb;
                 o[0] += st * (ai - s1[t]);
                 o[1] += st * (ci - s2[t]);
             } else {
-                const dual::D ft = dual::xy_diff_x(dxo, dyo);
+                // (d xy / dx is even, so it comes from the same orientation)
+                dual::D fv, ft;
+                dual::both(dxo, dyo, fv, ft);
                 const double st = ft.v * bb, tt = (lo ? ft.d : -ft.d) * bb;
+                const double sp = fv.d * bb;
                 if (kMode == kModeJvp) {
-                    const double sp = dual::xy(dx, dy).d * bb;
                     const double da = ai - s1[t];
                     o[0] += sp * da;
                     o[1] += tt * da;
@@ -149,7 +164,6 @@ __global__ void __launch_bounds__(kPT) k_deriv(DerivArgs A, double *part) {
                     o[4] += st * (qi - s2[t]);
                     o[5] += st * (ri - s3[t]);
                 } else {
-                    const double sp = dual::xy(dx, dy).d * bb;
                     o[0] += sp * (ai - s1[t]) +
                             tt * ((pi - s2[t]) * (qi - s3[t]) + (ri - s4[t]) * (si - s5[t]) +
                                   (ui + s6[t]));
@@ -164,26 +178,34 @@ __global__ void __launch_bounds__(kPT) k_deriv(DerivArgs A, double *part) {
     for (int k = 0; k < nout; ++k) part[((size_t)k * gridDim.y + blockIdx.y) * n + i] = o[k];
 }
 
-__global__ void k_deriv_sum(int n, int tiles, int nout, const double *part, DerivArgs A) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    for (int k = 0; k < nout; ++k) {
-        double v = 0;
-        for (int t = 0; t < tiles; ++t) v += part[((size_t)k * tiles + t) * n + i];
-        A.o[k][i] = v;
-    }
+// One output of 32 rows per block: kSumWarps warps add every kSumWarps-th tile,
+// the first then adds the warps' sums in order.
+constexpr int kSumWarps = 8;
+__global__ void __launch_bounds__(32 * kSumWarps)
+    k_deriv_sum(int n, int tiles, const double *part, DerivArgs A) {
+    __shared__ double sum[kSumWarps][32];
+    const int i = blockIdx.x * 32 + threadIdx.x, k = blockIdx.y;
+    double v = 0;
+    if (i < n)
+        for (int t = threadIdx.y; t < tiles; t += kSumWarps)
+            v += part[((size_t)k * tiles + t) * n + i];
+    sum[threadIdx.y][threadIdx.x] = v;
+    __syncthreads();
+    if (threadIdx.y || i >= n) return;
+    for (int w = 1; w < kSumWarps; ++w) v += sum[w][threadIdx.x];
+    A.o[k][i] = v;
 }
 
-// Launches k_deriv<kMode> over all pair tiles and the in-order tile sum.
+// Launches k_deriv<kMode> over all pair tiles and the sum over the tiles.
 template <int kMode>
 void run_deriv(Ctx &c, DerivArgs &A, double *part) {
-    const int tiles = nb(c.n, kPT);
+    const int tiles = nb(c.n, cols_per_block(c.n));
     const int nout = (kMode == kModeJv || kMode == kModeJt) ? (A.o[1] ? 2 : 1)
                      : kMode == kModeJvp                   ? 6
                                                            : 1;
-    k_deriv<kMode><<<dim3(tiles, tiles), kPT, 0, c.stream>>>(A, part);
+    k_deriv<kMode><<<dim3(nb(c.n, kPT), tiles), kPT, 0, c.stream>>>(A, part);
     check_launch("k_deriv");
-    k_deriv_sum<<<nb(c.n, 256), 256, 0, c.stream>>>(c.n, tiles, nout, part, A);
+    k_deriv_sum<<<dim3(nb(c.n, 32), nout), dim3(32, kSumWarps), 0, c.stream>>>(c.n, tiles, part, A);
     check_launch("k_deriv_sum");
 }
 
@@ -566,7 +588,7 @@ int d4_tangent(void *ctx, long long steps, const double *t0s, const double *hs,
                                    c->stream));
         double *dz = w.alloc(n), *dzs = w.alloc(n), *dx1 = w.alloc(n), *dd = w.alloc(n),
                *rhs = w.alloc(n), *jx1 = w.alloc(n);
-        double *part = w.alloc((size_t)6 * nb(n, kPT) * n);
+        double *part = w.alloc((size_t)6 * nb(n, cols_per_block(n)) * n);
         double *o[6];
         for (double *&p : o) p = w.alloc(n);
         D4_CUDA_OK(cudaMemcpyAsync(dz, dx0, sizeof(double) * n, cudaMemcpyHostToDevice,
@@ -654,7 +676,7 @@ int d4_adjoint(void *ctx, long long steps, const double *t0s, const double *hs,
                *dmu = w.alloc(n), *w1 = w.alloc(n), *lx1 = w.alloc(n), *jd1 = w.alloc(n),
                *jd2 = w.alloc(n), *ea = w.alloc(n), *eq = w.alloc(n), *es = w.alloc(n),
                *eu = w.alloc(n), *oz = w.alloc(n);
-        double *part = w.alloc((size_t)6 * nb(n, kPT) * n);
+        double *part = w.alloc((size_t)6 * nb(n, cols_per_block(n)) * n);
         D4_CUDA_OK(cudaMemsetAsync(lam_next, 0, sizeof(double) * n, c->stream));
         double *tsc = w.alloc(n);  // forward-pass result of the transposed solves
         for (long long seg = nseg - 1; seg >= 0; --seg) {

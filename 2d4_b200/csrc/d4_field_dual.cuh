@@ -49,12 +49,20 @@ __device__ __forceinline__ D dsinh(D x) { return D{sinh(x.v), cosh(x.v) * x.d}; 
 
 using f64::kPi;
 
+// Quotients of the images (divisors far inside the normal range): both parts from
+// one reciprocal, correctly rounded as a division's (d4_field64.cuh).
+__device__ __forceinline__ D ratio(D a, D b) {
+    const double y = f64::recip(b.v);
+    const double q = f64::quot(a.v, b.v, y);
+    return D{q, f64::quot(a.d - q * b.d, b.v, y)};
+}
+
 // Hyperbolic values of 2 pi (dx +- i) from e = exp(2 pi dx), as f64::Hyp.
 struct Hyp {
     D ch0, sh0, chp1, chm1, shp1, shm1, chp2, chm2, shp2, shm2;
     D chp3, chm3, chp4, chm4, chp5, chm5;
     __device__ __forceinline__ explicit Hyp(D e) {
-        const D inv = 1.0 / e;
+        const D inv = ratio(mk(1.0), e);
         const D s = e + inv, d = e - inv;
         ch0 = s / 2;
         sh0 = d / 2;
@@ -67,17 +75,17 @@ struct Hyp {
         shp2 = (d * f64::kCosh4Pi + s * f64::kSinh4Pi) / 2;
         shm2 = (d * f64::kCosh4Pi - s * f64::kSinh4Pi) / 2;
         chp3 = e * f64::kCosh6Pi;
-        chm3 = f64::kCosh6Pi / e;
+        chm3 = ratio(mk(f64::kCosh6Pi), e);
         chp4 = e * f64::kCosh8Pi;
-        chm4 = f64::kCosh8Pi / e;
+        chm4 = ratio(mk(f64::kCosh8Pi), e);
         chp5 = e * f64::kCoshTPi;
-        chm5 = f64::kCoshTPi / e;
+        chm5 = ratio(mk(f64::kCoshTPi), e);
     }
 };
 
 __device__ __forceinline__ D f_l(D dx, double c, D ch) {
     const D q = ch - c;
-    return dx * (2 * kPi) * (ch * c - 1) / (q * q) * kPi;
+    return ratio(dx * (2 * kPi) * (ch * c - 1), q * q) * kPi;
 }
 
 __device__ __forceinline__ D f_dx_l(D dx, double c, D ch, D sh) {
@@ -85,7 +93,8 @@ __device__ __forceinline__ D f_dx_l(D dx, double c, D ch, D sh) {
     const D q = ch - c;
     const D n1 = ch * c - 1;
     const D q2 = q * q;
-    return (n1 / q2 + dx2pi * (sh * c / q2 - n1 / (q2 * q) * 2 * sh)) * (2 * kPi * kPi);
+    return (ratio(n1, q2) + dx2pi * (ratio(sh * c, q2) - ratio(n1, q2 * q) * 2 * sh)) *
+           (2 * kPi * kPi);
 }
 
 // Taylor branch of f_dx_0 (dx^2 + dy^2 <= 1e-6), Field.cpp:224-249.
@@ -136,36 +145,46 @@ __device__ __forceinline__ Hyp hyp_of(double dxv) {
 }
 
 // {Field::xy(dx, dy), its derivative in dx} (Field.cpp:295-311).
-__device__ __forceinline__ D xy(double dxv, double dy) {
+__device__ __forceinline__ D xy(const Hyp &h, double c, double dxv, double dy) {
     const D dx = mk(dxv, 1.0);
-    const Hyp h = hyp_of(dxv);
-    const double c = cos(kPi * 2 * dy);
     const D g3 = f_l(dx + 3, c, h.chp3) + f_l(dx - 3, c, h.chm3) + f_l(dx + 2, c, h.chp2) +
                  f_l(dx - 2, c, h.chm2) + f_l(dx + 1, c, h.chp1) + f_l(dx - 1, c, h.chm1) +
                  f_0(dx, c, dy, h.ch0);
-    if (dxv < 0)
-        return f_l(dx + 5, c, h.chp5) * (0 - dx) + f_l(dx - 4, c, h.chm4) * (1 + dx) +
-               f_l(dx + 4, c, h.chp4) + g3;
-    return f_l(dx - 5, c, h.chm5) * dx + f_l(dx + 4, c, h.chp4) * (1 - dx) +
-           f_l(dx - 4, c, h.chm4) + g3;
+    // the blended images -+5 and -+4 (the pair's far side), then +-4
+    const bool neg = dxv < 0;
+    const double sg = neg ? -1.0 : 1.0;
+    const D far = dx * sg;
+    return f_l(dx - 5 * sg, c, neg ? h.chp5 : h.chm5) * far +
+           f_l(dx + 4 * sg, c, neg ? h.chm4 : h.chp4) * (1 - far) +
+           f_l(dx - 4 * sg, c, neg ? h.chp4 : h.chm4) + g3;
+}
+__device__ __forceinline__ D xy(double dxv, double dy) {
+    return xy(hyp_of(dxv), cos(kPi * 2 * dy), dxv, dy);
 }
 
 // {Field::xy_diff_x(dx, dy), its derivative in dx}.
-__device__ __forceinline__ D xy_diff_x(double dxv, double dy) {
+__device__ __forceinline__ D xy_diff_x(const Hyp &h, double c, double dxv, double dy) {
     const D dx = mk(dxv, 1.0);
-    const Hyp h = hyp_of(dxv);
-    const double c = cos(kPi * 2 * dy);
     const D g3 = f_dx_0(dx, c, dy, h.ch0, h.sh0) + f_dx_l(dx + 1, c, h.chp1, h.shp1) +
                  f_dx_l(dx - 1, c, h.chm1, h.shm1) + f_dx_l(dx + 2, c, h.chp2, h.shp2) +
                  f_dx_l(dx - 2, c, h.chm2, h.shm2) + f_dx_l(dx + 3, c, h.chp3, h.chp3) +
                  f_dx_l(dx - 3, c, h.chm3, h.chm3);
-    if (dxv < 0)
-        return f_dx_l(dx + 5, c, h.chp5, h.chp5) * (0 - dx) - f_l(dx + 5, c, h.chp5) +
-               f_dx_l(dx - 4, c, h.chm4, h.chm4) * (1 + dx) + f_l(dx - 4, c, h.chm4) +
-               f_dx_l(dx + 4, c, h.chp4, h.chp4) + g3;
-    return f_dx_l(dx - 5, c, h.chm5, h.chm5) * dx + f_l(dx - 5, c, h.chm5) +
-           f_dx_l(dx + 4, c, h.chp4, h.chp4) * (1 - dx) - f_l(dx + 4, c, h.chp4) +
-           f_dx_l(dx - 4, c, h.chm4, h.chm4) + g3;
+    const bool neg = dxv < 0;
+    const double sg = neg ? -1.0 : 1.0;
+    const D far = dx * sg, ch5 = neg ? h.chp5 : h.chm5, ch4b = neg ? h.chm4 : h.chp4,
+            ch4 = neg ? h.chp4 : h.chm4;
+    return f_dx_l(dx - 5 * sg, c, ch5, ch5) * far + f_l(dx - 5 * sg, c, ch5) * sg +
+           f_dx_l(dx + 4 * sg, c, ch4b, ch4b) * (1 - far) - f_l(dx + 4 * sg, c, ch4b) * sg +
+           f_dx_l(dx - 4 * sg, c, ch4, ch4) + g3;
+}
+
+// Both at one (dx, dy), sharing the exponential, the cosine and the images'
+// common factors.
+__device__ __forceinline__ void both(double dxv, double dy, D &f, D &g) {
+    const Hyp h = hyp_of(dxv);
+    const double c = cos(kPi * 2 * dy);
+    f = xy(h, c, dxv, dy);
+    g = xy_diff_x(h, c, dxv, dy);
 }
 
 }  // namespace dual
