@@ -84,15 +84,15 @@ struct Args {
 };
 
 struct Smem {
-    double lp[2][2][NB][kBoxR];     // [buffer][row box]: a tile's L21 piece
-    double up[2][2][NB][kBoxC];     // [buffer][column box]: its U12 piece
-    double at[2][2][kBoxC][kBoxR];  // [row box][column box]: the next tile's entries
+    double lp[2][2][NB][kBoxR];     // [team][buffer]: a tile's L21 piece
+    double up[2][2][2][NB][kBoxC];  // [team][buffer][column box]: its U12 piece
+    double at[2][2][kBoxC][kBoxR];  // [team][column box]: the next tile's entries
     double s[NB][NB + 1];           // diagonal block (rows = positions k0..k0+31)
     double q[NB][NB + 1];           // its pre-division values
     double rs[NB];                  // RN(1 / pivot); 0 outside the quotient window
     double lcol[NB][NB];            // elimination: multipliers of each column
     uint64_t done[NB];              // elimination: mbarrier of each column
-    uint64_t full[2];               // update: a buffer's copies have landed
+    uint64_t full[2][2];            // update: [team][buffer]: the copies have landed
     double red_v[kWarps];
     int red_i[kWarps];
     int sa[NB], sb[NB];             // swap list of the block (positions)
@@ -105,6 +105,7 @@ struct Smem {
     unsigned la_mask;               // look-ahead: flags of the published diagonal block
 };
 static_assert(offsetof(Smem, up) % 128 == 0 && offsetof(Smem, at) % 128 == 0, "alignment");
+static_assert(sizeof(Smem) <= 227 * 1024, "shared memory of a CTA");
 
 // The CTA's shared memory.  Every function names it itself: through a reference
 // parameter the out-of-line ones would use generic loads (the rows' chain took
@@ -594,21 +595,18 @@ __device__ __forceinline__ void tile_at(int t, int tr, int tc, int &ti, int &tj)
     }
 }
 
-// Tiles of the update behind a block for a group of G CTAs.  128 x 64 from
-// three per CTA on (8 x 4 entries per thread: 0.94 of the product-difference
-// rate in a bare loop, 0.86 with 4 x 4); 64 x 32 when every CTA gets at most
-// one, where the tile's time is on the chain of the blocks; 64 x 64 between.
+// Tiles of the update behind a block for a group of G CTAs: 64 x 64 by each of two
+// teams per CTA; 64 x 32 by the whole CTA when every CTA gets at most one, where
+// the tile's time is on the chain of the blocks.
 struct Tiling {
-    int rm, rn;      // rows and columns per thread; a tile is 16 rm x 16 rn
+    int teams;       // teams of a CTA
     int tr, tc;      // tiles along rows and columns
     int la_tiles;    // tiles a CTA finishes in the time of a look-ahead
     __device__ Tiling(int rest, int G) {
-        const int t64 = (rest + 63) / 64;
-        rm = t64 * t64 >= 6 * (G - 1) && G > 1 ? 8 : 4;
-        rn = 2 * t64 * t64 <= G - 1 ? 2 : 4;
-        la_tiles = rm == 8 ? 3 : 5;
-        tr = (rest + 16 * rm - 1) / (16 * rm);
-        tc = (rest + 16 * rn - 1) / (16 * rn);
+        tr = (rest + kBoxR - 1) / kBoxR;
+        teams = 2 * tr * tr <= max(G - 1, 2) ? 1 : 2;
+        tc = teams == 2 ? tr : (rest + kBoxC - 1) / kBoxC;
+        la_tiles = 7;
     }
     __device__ int strips() const { return tr + tc - 1; }
 };
@@ -680,7 +678,7 @@ static __device__ __noinline__ void look_ahead(const Args &a, int k0, int kb, in
     Smem &S = smem();
     const int n = a.n, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     const int nk0 = k0 + NB, nkw = min(NB, n - nk0);
-    double *Lp = &S.lp[0][0][0][0], *Up = &S.up[0][0][0][0];
+    double *Lp = &S.lp[0][0][0][0], *Up = &S.up[0][0][0][0][0];
     double c[4] = {0, 0, 0, 0};
     for (int t = tid; t < NB * NB; t += kThreads) {
         const int r = t % NB, k = t / NB;
@@ -699,48 +697,71 @@ static __device__ __noinline__ void look_ahead(const Args &a, int k0, int kb, in
     publish(a, c, nk0, nkw, kb, pass);
 }
 
-// Trailing update: tiles first, first + stride, ... below `end`, 16 RM rows x
-// 16 RN columns.  Warp (wr, wc) of 2 x 4 owns 8 RM x 4 RN entries, lane (lr, lc)
-// of 8 x 4 the row pairs 2 lr + 16 p and column pairs 2 lc + 8 q of them, so
-// every operand is read as 16-byte words without bank conflicts.  The next
-// tile's L21 and U12 pieces and entries of A come by tensor copies of 64 x 32
-// boxes (one thread issues them) while a tile computes; as 16-byte cp.async by
-// every thread the issue alone held up each 128 x 64 tile 3,800 cycles of
-// 15,300, as untiled bulk copies of whole columns 8,600 on the issuing warp.
-// `seq` counts the CTA's tiles (buffer and mbarrier phase).  The tiles of the
-// first row also store U12 to A; tiles of the first column hold the next
-// block's columns, whose new values go to P0 instead of A.
-template <int RM, int RN>
-static __device__ __noinline__ unsigned update_tiles(const Args &a, int k0, int kb, const double *U,
+// Trailing update: tiles first, first + stride, ... below `end`.  A team is all
+// warps (64 x 32 tiles), or each half of them (64 x 64 tiles, team 1 takes every
+// second one): then one team's waits, loads and stores run under the other's
+// products.  The two take turns at the products (named barriers 3 and 4); left to
+// themselves they fall in step and stand still together.  N=4096: 128 x 64 tiles by
+// all warps 5.70 ms, two teams in step 5.61, in turns 5.15, with the operands of a
+// step fetched during the step before 5.02 (the products alone: 2.6).  Four teams
+// with 8 x 8 entries per thread and A read directly, in turns: 5.9 and more.
+// A warp owns 8 RM x 4 RN entries, lane (lr, lc) of 8 x 4 the row pairs 2 lr + 16 p
+// and column pairs 2 lc + 8 q of them, so every operand is read as 16-byte words
+// without bank conflicts (8 x 4 entries per thread in the teams: in a bare loop 0.96
+// of the product-difference rate by 8 warps, 0.88 by one team's 4; 4 x 4 0.91 and
+// 0.69).  The next tile's L21 and U12 pieces and entries of A come by tensor copies
+// of 64 x 32 boxes while a tile computes; as 16-byte cp.async by every thread the
+// issue alone held up 128 x 64 entries 3,800 cycles of 15,300, as untiled bulk copies
+// of whole columns 8,600 on the issuing warp.  `seq` counts the team's tiles (buffer
+// and mbarrier phase).  The tiles of the first row also store U12 to A; tiles of the
+// first column hold the next block's columns, whose new values go to P0, not A.
+template <int kTeams>
+static __device__ __noinline__ void update_tiles(const Args &a, int k0, int kb, const double *U,
                                               int ntr, int ntc, int first, int stride, int end,
                                               unsigned seq) {
     Smem &S = smem();
-    constexpr int kTr = 16 * RM, kTc = 16 * RN;
-    const int n = a.n, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    constexpr int RM = 4 * kTeams, RN = 2 * kTeams, kTr = kBoxR, kTc = 32 * kTeams,
+                  kTeam = kThreads / kTeams;
+    const int team = kTeams > 1 ? threadIdx.x / kTeam : 0;
+    const int n = a.n, tid = threadIdx.x % kTeam, warp = tid >> 5, lane = tid & 31;
+    auto sync = [&] {
+        if (kTeams > 1)
+            named_bar(1 + team, kTeam);
+        else
+            __syncthreads();
+    };
+    uint64_t *full = S.full[team];
     const int base = k0 + NB;
-    const int lr = (warp & 1) * 8 * RM + 2 * (lane & 7), lc = (warp >> 1) * 4 * RN + 2 * (lane >> 3);
-    const int rbox = lr / kBoxR, cbox = lc / kBoxC;
+    constexpr int kWr = kTr / (8 * RM);  // warps along a tile's rows
+    const int lr = warp % kWr * 8 * RM + 2 * (lane & 7), lc = warp / kWr * 4 * RN + 2 * (lane >> 3);
+    const int cbox = lc / kBoxC;
+    // warp 0 fetches the L21 piece, warp 1 U12's, the next ones the entries' (a copy's
+    // issue holds up its warp for some 300 cycles)
     auto stage = [&](int tile, unsigned buf) {
-        constexpr int kRb = (kTr + kBoxR - 1) / kBoxR, kCb = kTc / kBoxC;
+        constexpr int kCb = kTc / kBoxC;
+        if (lane != 0) return;
         int ti, tj;
         tile_at(tile, ntr, ntc, ti, tj);
         const int i0 = base + ti * kTr, j0 = base + tj * kTc;
-        uint64_t *bar = &S.full[buf];
-        bulk::arrive_expect_tx(bar, (uint32_t)sizeof(double) *
-                                        (kRb * NB * kBoxR + kCb * NB * kBoxC +
-                                         kRb * kCb * kBoxR * kBoxC));
-#pragma unroll
-        for (int r = 0; r < kRb; ++r) box_load(S.lp[buf][r], a.map_a, i0 + r * kBoxR, k0, bar);
-#pragma unroll
-        for (int c = 0; c < kCb; ++c)
-            box_load(S.up[buf][c], a.map_u, j0 + c * kBoxC, U == a.U ? 0 : NB, bar);
-#pragma unroll
-        for (int r = 0; r < kRb; ++r)
+        uint64_t *bar = &full[buf];
+        if (warp == 0) {
+            bulk::arrive_expect_tx(bar, (uint32_t)sizeof(double) *
+                                            (NB * kBoxR + kCb * NB * kBoxC + kCb * kBoxR * kBoxC));
+            box_load(S.lp[team][buf], a.map_a, i0, k0, bar);
+        } else if (warp == 1) {
 #pragma unroll
             for (int c = 0; c < kCb; ++c)
-                box_load(S.at[r][c], a.map_a, i0 + r * kBoxR, j0 + c * kBoxC, bar);
+                box_load(S.up[team][buf][c], a.map_u, j0 + c * kBoxC, U == a.U ? 0 : NB, bar);
+        } else if (warp < 2 + kCb) {
+            const int c = warp - 2;
+            box_load(S.at[team][c], a.map_a, i0, j0 + c * kBoxC, bar);
+        }
     };
-    if (tid == 0 && first < end) {
+    const int step = stride;  // from a tile to that of the other team's next turn
+    bool wait_turn = kTeams > 1 && team;
+    first += team * stride;
+    stride *= kTeams;
+    if (first < end) {
         fence_bulk();
         stage(first, seq & 1);
     }
@@ -749,10 +770,10 @@ static __device__ __noinline__ unsigned update_tiles(const Args &a, int k0, int 
         tile_at(tile, ntr, ntc, ti, tj);
         const int i0 = base + ti * kTr, j0 = base + tj * kTc;
         const unsigned buf = seq & 1;
-        const double *Ls = &S.lp[buf][rbox][0][lr % kBoxR];
-        const double *Us = &S.up[buf][cbox][0][lc % kBoxC];
-        const double *At = &S.at[rbox][cbox][lc % kBoxC][lr % kBoxR];
-        if (!bulk::wait(&S.full[buf], (seq >> 1) & 1)) atomicOr(&a.flags[kFlagBarrierTimeout], 1);
+        const double *Ls = &S.lp[team][buf][0][lr];
+        const double *Us = &S.up[team][buf][cbox][0][lc % kBoxC];
+        const double *At = &S.at[team][cbox][lc % kBoxC][lr];
+        if (!bulk::wait(&full[buf], (seq >> 1) & 1)) atomicOr(&a.flags[kFlagBarrierTimeout], 1);
         double acc[RN][RM];  // [column][row]
 #pragma unroll
         for (int q = 0; q < RN; ++q)
@@ -763,28 +784,41 @@ static __device__ __noinline__ unsigned update_tiles(const Args &a, int k0, int 
                 acc[q][2 * p] = v.x;
                 acc[q][2 * p + 1] = v.y;
             }
-        __syncthreads();  // the entries are in registers; the other buffer is free
-        if (tid == 0 && tile + stride < end) stage(tile + stride, buf ^ 1);
-#pragma unroll 2
-        for (int k = 0; k < NB; ++k) {
-            double lv[RM], uv[RN];
+        sync();  // the entries are in registers; the other buffer is free
+        if (tile + stride < end) stage(tile + stride, buf ^ 1);
+        if (kTeams > 1 && wait_turn) named_bar(3 + team, kThreads);
+        wait_turn = true;
+        double lv[2][RM], uv[2][RN];
+        auto fetch = [&](int k, double (&l)[RM], double (&u)[RN]) {
 #pragma unroll
             for (int p = 0; p < RM / 2; ++p) {
                 const double2 v = *reinterpret_cast<const double2 *>(Ls + k * kBoxR + 16 * p);
-                lv[2 * p] = v.x;
-                lv[2 * p + 1] = v.y;
+                l[2 * p] = v.x;
+                l[2 * p + 1] = v.y;
             }
 #pragma unroll
             for (int q = 0; q < RN / 2; ++q) {
                 const double2 v = *reinterpret_cast<const double2 *>(Us + k * kBoxC + 8 * q);
-                uv[2 * q] = v.x;
-                uv[2 * q + 1] = v.y;
+                u[2 * q] = v.x;
+                u[2 * q + 1] = v.y;
             }
+        };
+        auto products = [&](const double (&l)[RM], const double (&u)[RN]) {
 #pragma unroll
             for (int q = 0; q < RN; ++q)
 #pragma unroll
-                for (int p = 0; p < RM; ++p) acc[q][p] = acc[q][p] - lv[p] * uv[q];
+                for (int p = 0; p < RM; ++p) acc[q][p] = acc[q][p] - l[p] * u[q];
+        };
+        fetch(0, lv[0], uv[0]);
+#pragma unroll 4
+        for (int k = 0; k < NB; k += 2) {
+            fetch(k + 1, lv[1], uv[1]);
+            products(lv[0], uv[0]);
+            fetch((k + 2) % NB, lv[0], uv[0]);
+            products(lv[1], uv[1]);
         }
+        if (kTeams > 1 && tile + step < end)  // the other team's turn
+            asm volatile("bar.arrive %0, %1;" ::"r"(4 - team), "r"(kThreads) : "memory");
 #pragma unroll
         for (int q = 0; q < RN; q += 2) {
             const int lj = lc + 4 * q, gj = j0 + lj;
@@ -807,15 +841,16 @@ static __device__ __noinline__ unsigned update_tiles(const Args &a, int k0, int 
         }
         // products done with this buffer before it is refilled; a strip tile's
         // stores are in before it is counted
-        __syncthreads();
-        if (tile < ntr + ntc - 1 && tid == kThreads - 1) red_rel(a.sched + kb, 1u);
+        sync();
+        if (tile < ntr + ntc - 1 && tid == kTeam - 1) red_rel(a.sched + kb, 1u);
         if (ti == 0) {
             // U12 to A, from this buffer (not refilled before the next barrier)
 #pragma unroll
-            for (int r = 0; r < NB * kTc / 2 / kThreads; ++r) {
-                const int t = tid + r * kThreads, k = t % NB, jj = 2 * (t / NB);
+            for (int r = 0; r < NB * kTc / 2 / kTeam; ++r) {
+                const int t = tid + r * kTeam, k = t % NB, jj = 2 * (t / NB);
                 if (j0 + jj < n) {
-                    const double2 v = *reinterpret_cast<const double2 *>(&S.up[buf][jj / kBoxC][k][jj % kBoxC]);
+                    const double2 v = *reinterpret_cast<const double2 *>(
+                        &S.up[team][buf][jj / kBoxC][k][jj % kBoxC]);
                     double *dst = a.A + (size_t)(k0 + k) + (size_t)(j0 + jj) * n;
                     dst[0] = v.x;
                     dst[n] = v.y;
@@ -823,7 +858,6 @@ static __device__ __noinline__ unsigned update_tiles(const Args &a, int k0, int 
             }
         }
     }
-    return seq;
 }
 
 template <class Group>
@@ -839,7 +873,7 @@ __device__ __forceinline__ void factor(const Args &a, Group g) {
     if (tid < NB)
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&S.done[tid]))
                      : "memory");
-    if (tid < 2) bulk::init(&S.full[tid], 1);
+    if (tid < 4) bulk::init(&S.full[tid >> 1][tid & 1], 1);
     bulk::fence_init();
     for (int i = cta * kThreads + tid; i < n; i += G * kThreads) a.perm[i] = i;
     // P0 = the first block's columns
@@ -852,7 +886,7 @@ __device__ __forceinline__ void factor(const Args &a, Group g) {
 
     const int Gt = G > 1 ? G - 1 : 1;  // CTAs that take rows, columns and most tiles
     int swaps = 0;  // row swaps so far
-    unsigned seq = 0;  // update tiles of this CTA so far
+    unsigned seq0 = 0, seq1 = 0;  // update tiles of this CTA's teams so far
     int pass = 0;   // pass counter: mask word, and Q buffer by parity
     for (int kb = 0; kb < nblk; ++kb) {
         const int k0 = kb * NB, kw = min(NB, n - k0), rest = n - k0 - kw;
@@ -919,7 +953,7 @@ __device__ __forceinline__ void factor(const Args &a, Group g) {
                 __syncthreads();
             }
             bool good = true;
-            double *Lp = &S.lp[0][0][0][0], *Up = &S.up[0][0][0][0];  // [k][row], [k][column]
+            double *Lp = &S.lp[0][0][0][0], *Up = &S.up[0][0][0][0][0];  // [k][row], [k][column]
             for (int t = spec ? warp : cta < Gt ? warp * Gt + cta : 2 * groups;
                  t < (spec ? kWarps : 2 * groups); t += spec ? kWarps : kWarps * Gt) {
                 // (the look-ahead has 2 NB / kRows tasks; its other warps pass by)
@@ -1105,12 +1139,16 @@ __device__ __forceinline__ void factor(const Args &a, Group g) {
                     end = tiles;
                 }
             }
-            if (T.rm == 8)
-                seq = update_tiles<8, 4>(a, k0, kb, U, T.tr, T.tc, first, stride, end, seq);
-            else if (T.rn == 4)
-                seq = update_tiles<4, 4>(a, k0, kb, U, T.tr, T.tc, first, stride, end, seq);
-            else
-                seq = update_tiles<4, 2>(a, k0, kb, U, T.tr, T.tc, first, stride, end, seq);
+            const int mine = end > first ? (end - first + stride - 1) / stride : 0;
+            if (T.teams == 2) {
+                update_tiles<2>(a, k0, kb, U, T.tr, T.tc, first, stride, end,
+                                tid < kThreads / 2 ? seq0 : seq1);
+                seq0 += (mine + 1) / 2;
+                seq1 += mine / 2;
+            } else {
+                update_tiles<1>(a, k0, kb, U, T.tr, T.tc, first, stride, end, seq0);
+                seq0 += mine;
+            }
         }
     }
     if (cta == 0 && tid == 0) {
