@@ -259,12 +259,21 @@ struct ProfScope {
 extern std::atomic<long long> g_launches;
 extern std::atomic<long long> g_allocs;
 
+// Frees the device block that the pattern analysis keeps between calls.
+void release_spare();
+
 // Every device allocation of the library goes through this wrapper, which
 // counts it (d4_device_allocations).
 template <typename T>
 inline cudaError_t dmalloc(T **p, size_t bytes) {
     g_allocs.fetch_add(1, std::memory_order_relaxed);
-    return cudaMalloc((void **)p, bytes);
+    cudaError_t e = cudaMalloc((void **)p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        release_spare();
+        e = cudaMalloc((void **)p, bytes);
+    }
+    return e;
 }
 
 // ---- FP64 pair sweeps (d4_fp64.cu) ----
