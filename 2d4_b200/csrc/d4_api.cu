@@ -832,7 +832,7 @@ int d4_create(void **out, int n, const d4_params *p) {
             dalloc(&c->m_conv, (size_t)d4::kIrMax + 1);
             dalloc(&c->m_c32, (size_t)n);
             dalloc(&c->m_w1, (size_t)n);
-            dalloc(&c->m_part, (size_t)((n + 255) / 256) * n);
+            dalloc(&c->m_part, (size_t)((n + d4::kResidCols - 1) / d4::kResidCols) * n);
             dalloc(&c->m_resid, 16);
             D4_CUDA_OK(cudaMemset(c->m_resid, 0, sizeof(unsigned long long) * 16));
             std::vector<int> ident(n);
@@ -931,7 +931,7 @@ int d4_create(void **out, int n, const d4_params *p) {
                 dalloc(&B.dx2, (size_t)n);
                 dalloc(&B.cnt, (size_t)(n + 255) / 256);
                 D4_CUDA_OK(cudaMemset(B.cnt, 0, sizeof(unsigned) * ((n + 255) / 256)));
-                dalloc(&B.part, (size_t)((n + 255) / 256) * n);
+                dalloc(&B.part, (size_t)((n + d4::kResidCols - 1) / d4::kResidCols) * n);
                 dalloc(&B.c32, (size_t)n);
                 dalloc(&B.w1, (size_t)n);
                 dalloc(&B.resid, 16);

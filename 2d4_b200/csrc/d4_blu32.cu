@@ -182,17 +182,35 @@ __device__ void store_tile(const Args &a, const float *Sp, int ti, int tj, bool 
     }
 }
 
+// 1 / d for a pivot: the approximation (within an ulp) and one Newton step.
+__device__ __forceinline__ float pivot_recip(float d) {
+    float p;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(p) : "f"(d));
+    return fmaf(p, fmaf(-d, p, 1.f), p);
+}
+__device__ __forceinline__ void ld8(const float *p, float (&v)[8]) {
+    const float4 a = *reinterpret_cast<const float4 *>(p), b = *reinterpret_cast<const float4 *>(p + 4);
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+    v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+}
+
 // In-place Gauss-Jordan inverse of the 128 x 128 tile in Sp (no pivoting):
 // thread (tr, tc) of a 16 x 16 grid keeps rows 8tr.. and columns 8tc.. in
 // registers.  The step of pivot k is the rank-1 form
 //     a_rc <- [c != k] a_rc - L_r U_c  (+1 at r = c = k)
 // with L_r = a_rk (a_kk - 1 at r = k) and U_c = a_kc / a_kk (1 / a_kk at
-// c = k).  Pivots go in pairs (k, k+1) with one block barrier per pair: the
+// c = k).  Pivots go in pairs (k, k+1) with one exchange per pair: the
 // owners publish columns k, k+1 and rows k, k+1 as they stand before pivot k
 // (double-buffered), and every thread forms column k+1 and row k+1 after
 // pivot k for its own rows and columns with the same products the owners
-// would use, so the result is the one-pivot-at-a-time inverse bit for bit.
-// Returns false (on thread 0) when a pivot is zero or not finite.
+// would use, so the result is the one-pivot-at-a-time inverse.
+// Bound by what a pair loads from shared memory (36 KB: 290 cycles), its updates
+// (256 cycles of FP32 issue) and the chain between them (two reciprocals), one after
+// the other: 810 cycles a pair, 910 with scalar loads and IEEE divisions.  The next
+// pair's rows and columns are updated and published before the other 36 entries of a
+// thread, whose updates run while the others arrive.
+// Returns false (on thread 0) when a pivot is zero, not finite or outside the
+// range of the reciprocal.
 __device__ bool gauss_jordan(float *Sp, float *cbuf, float *rbuf) {
     const int tid = threadIdx.x;
     const int tr = tid >> 4, tc = tid & 15;
@@ -202,83 +220,86 @@ __device__ bool gauss_jordan(float *Sp, float *cbuf, float *rbuf) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) a[i][j] = Sp[(8 * tr + i) * kSp + 8 * tc + j];
     bool ok = true;
+    // columns and rows nl, nl+1 of group nb, before their pivots, into buffer `buf`
+    auto publish = [&](int nb, int nl, int buf) {
+        float *cb = cbuf + buf * 2 * kB, *rb = rbuf + buf * 2 * kB;
+        if (tc == nb) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+#pragma unroll
+                for (int i = 0; i < 8; i += 4)
+                    *reinterpret_cast<float4 *>(cb + e * kB + 8 * tr + i) = make_float4(
+                        a[i][nl + e], a[i + 1][nl + e], a[i + 2][nl + e], a[i + 3][nl + e]);
+        }
+        if (tr == nb) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+#pragma unroll
+                for (int j = 0; j < 8; j += 4)
+                    *reinterpret_cast<float4 *>(rb + e * kB + 8 * tc + j) = make_float4(
+                        a[nl + e][j], a[nl + e][j + 1], a[nl + e][j + 2], a[nl + e][j + 3]);
+        }
+    };
+    publish(0, 0, 0);
     // pivots in groups of 8: the group index kb is a loop variable, the pair's
     // place kl inside the group is a compile-time index into the registers
 #pragma unroll 1
     for (int kb = 0; kb < kB / 8; ++kb)
 #pragma unroll
     for (int kl = 0; kl < 8; kl += 2) {
-        const int k = 8 * kb + kl;
-        float *cb = cbuf + ((kl >> 1) & 1) * 2 * kB;  // columns k, k+1
-        float *rb = rbuf + ((kl >> 1) & 1) * 2 * kB;  // rows k, k+1
-        if (tc == kb) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                cb[8 * tr + i] = a[i][kl];
-                cb[kB + 8 * tr + i] = a[i][kl + 1];
-            }
-        }
-        if (tr == kb) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                rb[8 * tc + j] = a[kl][j];
-                rb[kB + 8 * tc + j] = a[kl + 1][j];
-            }
-        }
+        const int k = 8 * kb + kl, buf = (kl >> 1) & 1;
+        const float *cb = cbuf + buf * 2 * kB;  // columns k, k+1
+        const float *rb = rbuf + buf * 2 * kB;  // rows k, k+1
+        const bool pc = tc == kb, pr = tr == kb;  // owners of the columns, of the rows
         __syncthreads();
+        const float2 d0 = *reinterpret_cast<const float2 *>(rb + k);       // a_kk, a_k,k+1
+        const float2 d1 = *reinterpret_cast<const float2 *>(rb + kB + k);  // a_k+1,k, a_k+1,k+1
+        float L[8], U[8], L2[8], U2[8];
+        ld8(cb + 8 * tr, L);
+        ld8(rb + 8 * tc, U);
+        ld8(cb + kB + 8 * tr, L2);
+        ld8(rb + kB + 8 * tc, U2);
         // ---- pivot k
-        const float akk = rb[k];
-        const float p = 1.0f / akk;
-        if (tid == 0 && !(isfinite(p) && akk != 0.f)) ok = false;
-        float L[8], U[8], C1[8], R1[8];
+        const float p = pivot_recip(d0.x);
+        const float uk1 = d0.y * p;              // U at column k+1
+        const float ak1 = fmaf(-d1.x, uk1, d1.y);  // a_{k+1,k+1} after pivot k
+        const float p2 = pivot_recip(ak1);
+        if (tid == 0 && !(isfinite(p) && p != 0.f && isfinite(p2) && p2 != 0.f)) ok = false;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) L[i] = cb[8 * tr + i];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) U[j] = rb[8 * tc + j] * p;
-        if (tc == kb) U[kl] = p;
-        if (tr == kb) L[kl] = akk - 1.f;
+        for (int j = 0; j < 8; ++j) U[j] *= p;
+        if (pc) U[kl] = p;
+        if (pr) L[kl] = d0.x - 1.f;
         // column k+1 (own rows) and row k+1 (own columns) after pivot k
-        const float uk1 = rb[k + 1] * p;  // U at column k+1
-        const float lk1 = rb[kB + k];     // L at row k+1: a_{k+1,k}
 #pragma unroll
-        for (int i = 0; i < 8; ++i) C1[i] = fmaf(-L[i], uk1, cb[kB + 8 * tr + i]);
+        for (int i = 0; i < 8; ++i) L2[i] = fmaf(-L[i], uk1, L2[i]);
+        if (pc) U2[kl] = 0.f;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const float r0 = rb[kB + 8 * tc + j];
-            R1[j] = (tc == kb && j == kl) ? -lk1 * U[j] : fmaf(-lk1, U[j], r0);
-        }
-        const float ak1 = fmaf(-lk1, uk1, rb[kB + k + 1]);  // a_{k+1,k+1} after pivot k
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                if (j == kl)
-                    a[i][j] = (tc == kb) ? -L[i] * U[j] : fmaf(-L[i], U[j], a[i][j]);
-                else
-                    a[i][j] = fmaf(-L[i], U[j], a[i][j]);
-            }
-        }
-        if (tr == kb && tc == kb) a[kl][kl] += 1.f;
+        for (int j = 0; j < 8; ++j) U2[j] = fmaf(-d1.x, U[j], U2[j]) * p2;
         // ---- pivot k+1
-        const float p2 = 1.0f / ak1;
-        if (tid == 0 && !(isfinite(p2) && ak1 != 0.f)) ok = false;
+        if (pc) U2[kl + 1] = p2;
+        if (pr) L2[kl + 1] = ak1 - 1.f;
+        auto update = [&](int i, int j) {
+            float v = a[i][j];
+            if (j == kl) v = pc ? 0.f : v;
+            v = fmaf(-L[i], U[j], v);
+            if (i == kl && j == kl) v = pc && pr ? v + 1.f : v;
+            if (j == kl + 1) v = pc ? 0.f : v;
+            v = fmaf(-L2[i], U2[j], v);
+            if (i == kl + 1 && j == kl + 1) v = pc && pr ? v + 1.f : v;
+            a[i][j] = v;
+        };
+        const int nl = (kl + 2) & 7;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) U[j] = R1[j] * p2;
-        if (tc == kb) U[kl + 1] = p2;
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) L[i] = C1[i];
-        if (tr == kb) L[kl + 1] = ak1 - 1.f;
+            for (int j = 0; j < 8; ++j)
+                if ((i & 6) == nl || (j & 6) == nl) update(i, j);
+        if (k + 2 < kB) publish(kl < 6 ? kb : kb + 1, nl, buf ^ 1);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                if (j == kl + 1)
-                    a[i][j] = (tc == kb) ? -L[i] * U[j] : fmaf(-L[i], U[j], a[i][j]);
-                else
-                    a[i][j] = fmaf(-L[i], U[j], a[i][j]);
-            }
-        }
-        if (tr == kb && tc == kb) a[kl + 1][kl + 1] += 1.f;
+            for (int j = 0; j < 8; ++j)
+                if ((i & 6) != nl && (j & 6) != nl) update(i, j);
     }
     __syncthreads();
 #pragma unroll

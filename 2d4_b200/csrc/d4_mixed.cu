@@ -91,69 +91,69 @@ __device__ __forceinline__ bool converged(const unsigned long long *conv, int do
 
 // One refinement sweep's update in one launch: dx_out = dx + c and
 // r = g - A dx_out with the FP64 matrix.  Block (x, y) multiplies rows 256x..
-// by column chunk y (FP64, column order, the chunk's corrected dx staged in
-// shared memory; the blocks of row block 0 also store it to dx_out, a buffer
-// no block reads) into part[y][i]; the last block of each row block to finish
+// (two per thread) by column chunk y (FP64, column order, the chunk's corrected dx
+// staged in shared memory; the blocks of row block 0 also store it to dx_out, a
+// buffer no block reads) into part[y][i]; the last block of each row block to finish
 // (a counter per row block, reset by that block) subtracts the chunk sums from
 // g in chunk order and adds its rows' max|r| to conv[it + 1].  The order of
 // every sum is fixed, so the residual is the same on every run.  When the
 // previous sweep already converged the launch only carries dx over.
-__global__ void __launch_bounds__(256) k_resid_fused(int n, const double *__restrict__ A,
-                                                     const double *__restrict__ dx,
-                                                     const float *__restrict__ corr,
-                                                     double *dx_out, const double *g,
-                                                     double *part, int chunk, int nch,
-                                                     unsigned *cnt, double *r,
-                                                     unsigned long long *conv, int it) {
-    __shared__ double sdx[256];
+// Bound by the read of A.  Chunks of kResidCols columns and 16-byte loads, 16 in
+// flight per thread: at n = 4096 1024 blocks, all resident, and 31 us for 134 MB
+// (chunks of 256 columns left 256 blocks, under two per SM: 88 us).
+constexpr int kResidThreads = kResidRows / 2;
+__global__ void __launch_bounds__(kResidThreads) k_resid_fused(
+    int n, const double *__restrict__ A, const double *__restrict__ dx,
+    const float *__restrict__ corr, double *dx_out, const double *g, double *part, int nch,
+    unsigned *cnt, double *r, unsigned long long *conv, int it) {
+    __shared__ double sdx[kResidCols];
     __shared__ int last;
-    const int c0 = blockIdx.y * chunk, c1 = min(n, c0 + chunk);
+    const int c0 = blockIdx.y * kResidCols, w = min(kResidCols, n - c0);
     if (converged(conv, it)) {
         if (blockIdx.x == 0)
-            for (int t = threadIdx.x; t < c1 - c0; t += blockDim.x) dx_out[c0 + t] = dx[c0 + t];
+            for (int t = threadIdx.x; t < w; t += kResidThreads) dx_out[c0 + t] = dx[c0 + t];
         if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
             atomicMax(conv + it + 1, __ldcg(conv + it));
         return;
     }
-    for (int t = threadIdx.x; t < c1 - c0; t += blockDim.x) {
+    for (int t = threadIdx.x; t < w; t += kResidThreads) {
         const double v = dx[c0 + t] + (double)corr[c0 + t];
         sdx[t] = v;
         if (blockIdx.x == 0) dx_out[c0 + t] = v;
     }
     __syncthreads();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = blockIdx.x * kResidRows + 2 * threadIdx.x;  // n is even
     if (i < n) {
-        // four interleaved sums (column c into sum c % 4), combined in a fixed
-        // order: independent FMA chains, and 16 loads issued together
-        const double *Ai = A + (size_t)i + (size_t)c0 * n;
-        const int w = c1 - c0;
-        double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
+        // four interleaved sums per row (column c into sum c % 4), combined in a
+        // fixed order: independent FMA chains
+        const double2 *Ai = reinterpret_cast<const double2 *>(A + (size_t)i + (size_t)c0 * n);
+        const size_t ld = n / 2;
+        double s[4][2] = {};
         int c = 0;
         for (; c + 16 <= w; c += 16) {
-            double av[16];
+            double2 av[16];
 #pragma unroll
-            for (int u = 0; u < 16; ++u) av[u] = __ldg(Ai + (size_t)(c + u) * n);
+            for (int u = 0; u < 16; ++u) av[u] = __ldg(Ai + (c + u) * ld);
 #pragma unroll
-            for (int u = 0; u < 16; u += 4) {
-                s0 += av[u] * sdx[c + u];
-                s1 += av[u + 1] * sdx[c + u + 1];
-                s2 += av[u + 2] * sdx[c + u + 2];
-                s3 += av[u + 3] * sdx[c + u + 3];
+            for (int u = 0; u < 16; ++u) {
+                s[u & 3][0] += av[u].x * sdx[c + u];
+                s[u & 3][1] += av[u].y * sdx[c + u];
             }
         }
-        for (; c < w; ++c) {
-            const double v = __ldg(Ai + (size_t)c * n) * sdx[c];
-            const int m = c & 3;
-            if (m == 0)
-                s0 += v;
-            else if (m == 1)
-                s1 += v;
-            else if (m == 2)
-                s2 += v;
-            else
-                s3 += v;
+        for (; c + 2 <= w; c += 2) {  // (w is even; c % 4 is 0 or 2)
+            const double2 v = __ldg(Ai + c * ld), u = __ldg(Ai + (c + 1) * ld);
+            const bool odd = c & 2;
+            s[0][0] += odd ? 0.0 : v.x * sdx[c];
+            s[0][1] += odd ? 0.0 : v.y * sdx[c];
+            s[1][0] += odd ? 0.0 : u.x * sdx[c + 1];
+            s[1][1] += odd ? 0.0 : u.y * sdx[c + 1];
+            s[2][0] += odd ? v.x * sdx[c] : 0.0;
+            s[2][1] += odd ? v.y * sdx[c] : 0.0;
+            s[3][0] += odd ? u.x * sdx[c + 1] : 0.0;
+            s[3][1] += odd ? u.y * sdx[c + 1] : 0.0;
         }
-        part[(size_t)blockIdx.y * n + i] = (s0 + s1) + (s2 + s3);
+        *reinterpret_cast<double2 *>(part + (size_t)blockIdx.y * n + i) = make_double2(
+            (s[0][0] + s[1][0]) + (s[2][0] + s[3][0]), (s[0][1] + s[1][1]) + (s[2][1] + s[3][1]));
     }
     __threadfence();
     __syncthreads();
@@ -163,10 +163,15 @@ __global__ void __launch_bounds__(256) k_resid_fused(int n, const double *__rest
     __threadfence();
     double a = 0;
     if (i < n) {
-        double v = g[i];
-        for (int q = 0; q < nch; ++q) v = v - __ldcg(part + (size_t)q * n + i);
-        r[i] = v;
-        a = fabs(v);
+        double2 v = *reinterpret_cast<const double2 *>(g + i);
+#pragma unroll 16
+        for (int q = 0; q < nch; ++q) {
+            const double2 p = __ldcg(reinterpret_cast<const double2 *>(part + (size_t)q * n + i));
+            v.x = v.x - p.x;
+            v.y = v.y - p.y;
+        }
+        *reinterpret_cast<double2 *>(r + i) = v;
+        a = nanmax(fabs(v.x), fabs(v.y));
     }
     if (threadIdx.x == 0) cnt[blockIdx.x] = 0;
     block_absmax(a, conv + it + 1);
@@ -352,12 +357,12 @@ static const float *solve32_once(Ctx &c, const Mix32Bufs &B, cudaStream_t st, co
 // alternates between B.dx and B.dx2, and a converged sweep only carries it
 // over, so after kIrMax launches the buffer is known on the host.  Returns it.
 static const double *refine(Ctx &c, const Mix32Bufs &B, cudaStream_t st) {
-    const int n = c.n, chunk = 256;
+    const int n = c.n, nch = nb(n, kResidCols);
     double *dxa = B.dx, *dxb = B.dx2;
     for (int it = 0; it < kIrMax; ++it) {
         const float *corr = solve32_once(c, B, st, B.r, it);
-        k_resid_fused<<<dim3(nb(n, 256), nb(n, chunk)), 256, 0, st>>>(
-            n, B.A64, dxa, corr, dxb, B.g, B.part, chunk, nb(n, chunk), B.cnt, B.r, B.conv, it);
+        k_resid_fused<<<dim3(nb(n, kResidRows), nch), kResidThreads, 0, st>>>(
+            n, B.A64, dxa, corr, dxb, B.g, B.part, nch, B.cnt, B.r, B.conv, it);
         check_launch("k_resid_fused");
         std::swap(dxa, dxb);
     }
