@@ -196,11 +196,11 @@ struct Ctx {
     // cutoff sparse path: CSR of the matrix and the GMRES work space
     int use_gmres = 0;
     int sp_grid = 0, sp_nch = 0, sp_cap = 0, sp_nnz = 0, sp_dense_ready = 0;
-    int *sp_cnt = nullptr, *sp_off = nullptr, *sp_rp = nullptr, *sp_ci = nullptr;
+    int *sp_off = nullptr, *sp_rp = nullptr, *sp_ci = nullptr;
     int *sp_flags = nullptr;
     unsigned *sp_bar = nullptr;
-    double *sp_val = nullptr, *sp_dinv = nullptr, *sp_V = nullptr, *sp_z = nullptr,
-           *sp_w = nullptr, *sp_g = nullptr, *sp_x = nullptr, *sp_part = nullptr;
+    double *sp_val = nullptr, *sp_dinv = nullptr, *sp_z = nullptr, *sp_x = nullptr,
+           *sp_part = nullptr;
     long long sp_solves = 0, sp_iters = 0, sp_fallbacks = 0;
     // cooperative LU counters (d4_lu_stats)
     long long lu_count = 0, lu_passes = 0, lu_swaps = 0;

@@ -7,8 +7,8 @@
 // as a CSC matrix (src/simulation.cpp:635-659).  Here the matrix is still
 // assembled densely by the pair kernels, so the row sums d_i and the row
 // scaling keep the reference's order, and is then compressed to CSR:
-//   k_csr_count  nonzeros per (row, 256-column chunk), one thread per row and chunk
-//   k_csr_rows   per-row chunk offsets and the row-pointer scan (one CTA)
+//   k_csr_count  nonzeros per (row, 256-column chunk), chunk offsets inside the rows
+//   k_csr_rows   the row-pointer scan (one CTA)
 //   k_csr_fill   column indices and values in ascending column order
 // Every solve of the step then runs GMRES(40) with right Jacobi preconditioning,
 // classical Gram-Schmidt with one reorthogonalisation and Givens rotations, to a
@@ -33,22 +33,24 @@ constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kStride = kM + 2;   // partials per CTA
 constexpr int kChunk = 256;       // columns per counting chunk
-constexpr int kGenWord = 32;
-constexpr long long kSpinLimit = 1ll << 24;  // polls of >= 64 ns: > 1 s
+constexpr int kCountChunks = 16;  // chunks counted at once
+constexpr int kSpLanes = 8;       // lanes per row of the SpMV
+constexpr int kRowsPer = 32;      // rows per CTA as long as the SMs suffice
+constexpr long long kSpinLimit = 1ll << 22;  // polls of several hundred cycles: > 1 s
 constexpr double kTol = 1e-13;
 
 struct GmresArgs {
     int n;
     const int *rp, *ci;
     const double *val, *dinv;
-    const double *g;  // right-hand side
-    double *x;        // solution (starts at 0)
-    double *V;        // (kM + 1) x n Krylov basis
-    double *z;        // n: preconditioned vector fed to the SpMV
-    double *w;        // n scratch
-    double *part;     // 2 x G x kStride partial sums
-    unsigned *bar;    // barrier words
-    int *flags;       // [0] barrier timeout, [1] not converged, [2] iterations
+    trsv::GArgs g;       // right-hand side
+    const double *base;  // out = base - x (out null: no output but dx)
+    double *out, *dx;    // written when the solve converged
+    double *x;           // n: the iterate
+    double *z;           // n: preconditioned vector fed to the SpMV
+    double *part;        // 2 x kStride x G partial sums
+    unsigned *bar;       // barrier counter (zeroed before the launch)
+    int *flags;          // [0] barrier timeout, [1] not converged, [2] iterations
 };
 
 __device__ __forceinline__ unsigned ld_acq(const unsigned *p) {
@@ -57,115 +59,123 @@ __device__ __forceinline__ unsigned ld_acq(const unsigned *p) {
     return v;
 }
 
-// Generation barrier over all CTAs.  The wait gives up after kSpinLimit polls
-// (or when another CTA gave up), sets flags[0] and marks the CTA dead, after
-// which it no longer waits; the host turns flags[0] into an error.
-__device__ void grid_barrier(unsigned *bar, int *flags, unsigned &gen, int *dead) {
+// Barrier over all CTAs (a counter that only grows).  The wait gives up after
+// kSpinLimit polls (or when another CTA gave up), sets flags[0] and marks the CTA
+// dead, after which it no longer waits; the host turns flags[0] into an error.
+__device__ __forceinline__ void grid_barrier(unsigned *bar, int *flags, unsigned &gen, int *dead) {
     __syncthreads();
     if (threadIdx.x == 0) {
-        const unsigned target = gen + 1;
-        __threadfence();
-        if (atomicAdd(bar, 1u) + 1 == gridDim.x) {
-            atomicExch(bar, 0u);
-            __threadfence();
-            atomicExch(bar + kGenWord, target);
-        } else if (!*dead) {
-            long long spins = 0;
-            while (ld_acq(bar + kGenWord) != target) {
-                __nanosleep(64);
-                if ((++spins & 255) == 0 &&
-                    (spins > kSpinLimit || ld_acq((const unsigned *)&flags[0]))) {
-                    atomicOr(&flags[0], 1);
-                    *dead = 1;
-                    break;
-                }
+        const unsigned target = ++gen * gridDim.x;
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+        long long spins = 0;
+        while (!*dead && (int)(ld_acq(bar) - target) < 0) {
+            if ((++spins & 255) == 0 &&
+                (spins > kSpinLimit || ld_acq((const unsigned *)&flags[0]))) {
+                atomicOr(&flags[0], 1);
+                *dead = 1;
             }
         }
-        gen = target;
     }
     __syncthreads();
 }
 
-// dst[i] = scale * sum_q val[q] * src[ci[q]] for the CTA's rows, one warp per row.
-__device__ __forceinline__ void spmv_rows(const GmresArgs &a, int r0, int r1, const double *src,
-                                          double scale, double *dst) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int i = r0 + wid; i < r1; i += kWarps) {
-        const int q0 = a.rp[i], q1 = a.rp[i + 1];
+// w[r] = scale * (A src)[r0 + r] for the CTA's rows, kSpLanes lanes per row.
+__device__ __forceinline__ void spmv_rows(const GmresArgs &a, int r0, int rows, const double *src,
+                                          double scale, double *w) {
+    const int l = threadIdx.x % kSpLanes;
+    for (int b = 0; b < rows; b += kThreads / kSpLanes) {
+        const int r = b + threadIdx.x / kSpLanes;
         double s = 0;
-        for (int q = q0 + lane; q < q1; q += 32) s += a.val[q] * __ldcg(src + a.ci[q]);
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) dst[i] = s * scale;
+        if (r < rows) {
+            const int q1 = a.rp[r0 + r + 1];
+#pragma unroll 4
+            for (int q = a.rp[r0 + r] + l; q < q1; q += kSpLanes)
+                s += a.val[q] * __ldcg(src + a.ci[q]);
+        }
+        for (int o = kSpLanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (l == 0 && r < rows) w[r] = s * scale;
     }
     __syncthreads();
 }
 
+// Bound by the three grid barriers of a Krylov vector (1.3 us each over 128 CTAs)
+// and the reductions around them.  32 rows per CTA, so that one pass of the SpMV
+// covers them with 8 lanes a row, the basis in shared memory (rows of a CTA only), a
+// warp per dot product and per total: N = 4096 486 -> 236 us a solve (128 rows per
+// CTA with one warp per row, the basis in memory, every total a serial sum, and a
+// sleeping barrier before).
 __global__ void __launch_bounds__(kThreads, 1) k_gmres(GmresArgs a) {
-    __shared__ double red[kWarps][kStride];
+    extern __shared__ double gm_smem[];
     __shared__ double H[kM + 1][kM];
-    __shared__ double tot[kStride], cs[kM], sn[kM], s[kM + 1], y[kM];
+    __shared__ double tot[kStride], hsum[kM], cs[kM], sn[kM], s[kM + 1], y[kM];
     __shared__ int dead, stop;
-    const int n = a.n, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int rows_per = (n + gridDim.x - 1) / gridDim.x;
-    const int r0 = min(n, (int)blockIdx.x * rows_per), r1 = min(n, r0 + rows_per);
+    const int n = a.n, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, G = gridDim.x;
+    const int rows_per = (n + G - 1) / G;
+    const int r0 = min(n, (int)blockIdx.x * rows_per), rows = min(n, r0 + rows_per) - r0;
+    double *V = gm_smem;                         // (kM + 1) x rows_per
+    double *w = V + (size_t)(kM + 1) * rows_per;  // rows_per
     unsigned gen = 0;
     int parity = 0;
     if (tid == 0) {
         dead = 0;
         stop = 0;
     }
-    __syncthreads();
-    double loc[kStride];
-    // Sum over all rows of loc[0..cnt) into tot[0..cnt): warp shuffles, per-warp
-    // rows in shared memory, one partial per CTA, grid barrier, then every CTA
-    // adds the partials in CTA order (identical totals everywhere).
-    auto reduce = [&](int cnt) {
-        double *P = a.part + (size_t)parity * gridDim.x * kStride;
-        for (int k = 0; k < cnt; ++k) {
-            double v = loc[k];
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-            if (lane == 0) red[wid][k] = v;
-        }
-        __syncthreads();
-        for (int k = tid; k < cnt; k += kThreads) {
+    // Sums over all rows of w times basis vector k (of w's square where `square`) into
+    // tot[0..cnt): a warp per sum over the CTA's rows, one partial per CTA, grid
+    // barrier, then a warp per total over the CTAs (identical totals everywhere).
+    auto reduce = [&](int cnt, bool square) {
+        double *P = a.part + (size_t)parity * G * kStride;
+        for (int k = wid; k < cnt; k += kWarps) {
+            const double *u = square ? w : V + (size_t)k * rows_per;
             double v = 0;
-            for (int q = 0; q < kWarps; ++q) v += red[q][k];
-            P[blockIdx.x * kStride + k] = v;
+            for (int r = lane; r < rows; r += 32) v += w[r] * u[r];
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0) P[(size_t)k * G + blockIdx.x] = v;
         }
         grid_barrier(a.bar, a.flags, gen, &dead);
-        for (int k = tid; k < cnt; k += kThreads) {
+        for (int k = wid; k < cnt; k += kWarps) {
             double v = 0;
-            for (int b = 0; b < (int)gridDim.x; ++b) v += __ldcg(P + b * kStride + k);
-            tot[k] = v;
+#pragma unroll 5
+            for (int b = lane; b < G; b += 32) v += __ldcg(P + (size_t)k * G + b);
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0) tot[k] = v;
         }
         __syncthreads();
         parity ^= 1;
     };
+    // w -= V tot over the basis vectors 0..j
+    auto subtract = [&](int j) {
+        if (tid < rows) {
+            double v = w[tid];
+            for (int k = 0; k <= j; ++k) v -= tot[k] * V[(size_t)k * rows_per + tid];
+            w[tid] = v;
+        }
+    };
     const int i = r0 + tid;  // the thread's row (rows_per <= kThreads)
-    const bool own = i < r1;
-    loc[0] = own ? a.g[i] * a.g[i] : 0;
-    reduce(1);
+    const bool own = tid < rows;
+    const double gi = own ? trsv::g_of(a.g, i) : 0, di = own ? a.dinv[i] : 0;
+    double xi = 0;
+    if (own) w[tid] = gi;
+    __syncthreads();
+    reduce(1, true);
     const double gnorm = sqrt(tot[0]);
     int iters = 0;
     bool converged = !(gnorm > 0);
     for (int cycle = 0; cycle < kRestarts && !converged && !dead; ++cycle) {
         // r = g - A x -> V_0, beta = ||r||
-        spmv_rows(a, r0, r1, a.x, 1.0, a.w);
-        double r = 0;
-        if (own) {
-            r = a.g[i] - a.w[i];
-            a.V[i] = r;
-        }
-        loc[0] = r * r;
-        reduce(1);
+        if (cycle > 0) spmv_rows(a, r0, rows, a.x, 1.0, w);
+        if (own) w[tid] = cycle > 0 ? gi - w[tid] : gi;
+        __syncthreads();
+        reduce(1, true);
         const double beta = sqrt(tot[0]);
         if (!(beta > kTol * gnorm)) {
             converged = true;
             break;
         }
         if (own) {
-            a.V[i] = r / beta;
-            a.z[i] = a.dinv[i] * (r / beta);
+            const double v = w[tid] / beta;
+            V[tid] = v;
+            a.z[i] = di * v;
         }
         if (tid == 0) {
             for (int k = 0; k <= kM; ++k) s[k] = 0;
@@ -176,27 +186,22 @@ __global__ void __launch_bounds__(kThreads, 1) k_gmres(GmresArgs a) {
         int jdone = 0;
         for (int j = 0; j < kM; ++j) {
             // w = A M^-1 V_j; first Gram-Schmidt pass
-            spmv_rows(a, r0, r1, a.z, 1.0 / zscale, a.w);
-            double w = own ? a.w[i] : 0;
-            for (int k = 0; k <= j; ++k) loc[k] = own ? w * a.V[(size_t)k * n + i] : 0;
-            reduce(j + 1);
-            double hsum[kM];
-            for (int k = 0; k <= j; ++k) hsum[k] = tot[k];
-            if (own)
-                for (int k = 0; k <= j; ++k) w -= tot[k] * a.V[(size_t)k * n + i];
+            spmv_rows(a, r0, rows, a.z, 1.0 / zscale, w);
+            reduce(j + 1, false);
+            subtract(j);
+            if (tid <= j) hsum[tid] = tot[tid];
+            __syncthreads();
             // reorthogonalisation
-            for (int k = 0; k <= j; ++k) loc[k] = own ? w * a.V[(size_t)k * n + i] : 0;
-            reduce(j + 1);
-            if (own)
-                for (int k = 0; k <= j; ++k) w -= tot[k] * a.V[(size_t)k * n + i];
-            for (int k = 0; k <= j; ++k) hsum[k] += tot[k];
+            reduce(j + 1, false);
+            subtract(j);
+            if (tid <= j) hsum[tid] += tot[tid];
             // ||w|| and the next (unnormalised) preconditioned vector share a barrier
-            if (own) a.z[i] = a.dinv[i] * w;
-            loc[0] = w * w;
-            reduce(1);
+            if (own) a.z[i] = di * w[tid];
+            __syncthreads();
+            reduce(1, true);
             const double nrm = sqrt(tot[0]);
             zscale = nrm > 0 ? nrm : 1.0;
-            if (own) a.V[(size_t)(j + 1) * n + i] = nrm > 0 ? w / nrm : 0;
+            if (own) V[(size_t)(j + 1) * rows_per + tid] = nrm > 0 ? w[tid] / nrm : 0;
             if (tid == 0) {
                 for (int k = 0; k <= j; ++k) H[k][j] = hsum[k];
                 for (int k = 0; k < j; ++k) {
@@ -229,12 +234,18 @@ __global__ void __launch_bounds__(kThreads, 1) k_gmres(GmresArgs a) {
         __syncthreads();
         if (own) {
             double u = 0;
-            for (int k = 0; k < jdone; ++k) u += y[k] * a.V[(size_t)k * n + i];
-            a.x[i] += a.dinv[i] * u;
+            for (int k = 0; k < jdone; ++k) u += y[k] * V[(size_t)k * rows_per + tid];
+            xi += di * u;
+            a.x[i] = xi;
         }
+        if (converged) break;
         grid_barrier(a.bar, a.flags, gen, &dead);
         if (tid == 0) stop = 0;
         __syncthreads();
+    }
+    if (own && converged && !dead) {
+        a.dx[i] = xi;
+        if (a.out) a.out[i] = a.base[i] - xi;
     }
     if (blockIdx.x == 0 && tid == 0) {
         if (!converged || dead) atomicOr(&a.flags[1], 1);
@@ -242,35 +253,46 @@ __global__ void __launch_bounds__(kThreads, 1) k_gmres(GmresArgs a) {
     }
 }
 
-// Nonzeros of row i in column chunk blockIdx.y (column-major matrix).
+// Nonzeros per (row, column chunk) of 32 rows per block, one thread per row and chunk,
+// 16 loads in flight (column-major matrix): chunk offsets off[ch][i] inside the row,
+// row totals to rp[i].
 template <typename T>
-__global__ void k_csr_count(int n, const T *__restrict__ A, int *cnt) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int ch = blockIdx.y;
-    if (i >= n) return;
-    const int j0 = ch * kChunk, j1 = min(n, j0 + kChunk);
-    int c = 0;
-    for (int j = j0; j < j1; ++j) c += A[(size_t)i + (size_t)j * n] != T(0);
-    cnt[(size_t)ch * n + i] = c;
+__global__ void __launch_bounds__(32 * kCountChunks) k_csr_count(int n, int nch,
+                                                                 const T *__restrict__ A,
+                                                                 int *__restrict__ off,
+                                                                 int *__restrict__ rp) {
+    __shared__ int cnt[kCountChunks][32];
+    const int i = blockIdx.x * 32 + threadIdx.x, y = threadIdx.y;
+    int run = 0;  // of the chunks before
+    for (int ch0 = 0; ch0 < nch; ch0 += kCountChunks) {
+        const int j0 = (ch0 + y) * kChunk, j1 = min(n, j0 + kChunk);
+        int c = 0;
+        if (i < n)
+#pragma unroll 16
+            for (int j = j0; j < j1; ++j) c += A[(size_t)i + (size_t)j * n] != T(0);
+        cnt[y][threadIdx.x] = c;
+        __syncthreads();
+        int before = run;
+        for (int q = 0; q < kCountChunks; ++q) {
+            if (q == y) before = run;
+            run += cnt[q][threadIdx.x];
+        }
+        if (i < n && ch0 + y < nch) off[(size_t)(ch0 + y) * n + i] = before;
+        __syncthreads();
+    }
+    if (i < n && y == 0) rp[i] = run;
 }
 
-// Per-row chunk offsets off[ch][i] and the row pointer rp[0..n] (one CTA of 1024).
-__global__ void __launch_bounds__(1024) k_csr_rows(int n, int nch, const int *cnt, int *off,
-                                                   int *rp) {
+// The row pointer rp[0..n] from the row totals in it (one CTA of 1024:
+// 5 us at n = 4096; 27 with the chunk offsets formed here too).
+__global__ void __launch_bounds__(1024) k_csr_rows(int n, int *rp) {
     __shared__ int part[1024];
     const int tid = threadIdx.x;
     const int per = (n + 1023) / 1024;
     const int b0 = min(n, tid * per), b1 = min(n, b0 + per);
     int sum = 0;
-    for (int i = b0; i < b1; ++i) {
-        int run = 0;
-        for (int ch = 0; ch < nch; ++ch) {
-            off[(size_t)ch * n + i] = run;
-            run += cnt[(size_t)ch * n + i];
-        }
-        rp[i] = run;  // row total for now
-        sum += run;
-    }
+#pragma unroll 4
+    for (int i = b0; i < b1; ++i) sum += rp[i];
     part[tid] = sum;
     __syncthreads();
     for (int o = 1; o < 1024; o <<= 1) {
@@ -288,40 +310,33 @@ __global__ void __launch_bounds__(1024) k_csr_rows(int n, int nch, const int *cn
     if (tid == 1023) rp[n] = part[1023];
 }
 
+// Bound by the read of A: 16 loads in flight per thread (134 MB at n = 4096: 47 us;
+// 73 with a load, a test and a store after each other).
 template <typename T>
-__global__ void k_csr_fill(int n, const T *__restrict__ A, const int *off, const int *rp, int *ci,
-                           double *val, double *dinv) {
+__global__ void k_csr_fill(int n, const T *__restrict__ A, const int *__restrict__ off,
+                           const int *__restrict__ rp, int *__restrict__ ci,
+                           double *__restrict__ val, double *__restrict__ dinv) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int ch = blockIdx.y;
     if (i >= n) return;
     const int j0 = ch * kChunk, j1 = min(n, j0 + kChunk);
     int q = rp[i] + off[(size_t)ch * n + i];
-    for (int j = j0; j < j1; ++j) {
-        const T v = A[(size_t)i + (size_t)j * n];
-        if (v != T(0)) {
-            ci[q] = j;
-            val[q] = (double)v;
-            ++q;
-        }
+    for (int jb = j0; jb < j1; jb += 16) {
+        T v[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) v[u] = jb + u < j1 ? A[(size_t)i + (size_t)(jb + u) * n] : T(0);
+#pragma unroll
+        for (int u = 0; u < 16; ++u)
+            if (v[u] != T(0)) {
+                ci[q] = jb + u;
+                val[q] = (double)v[u];
+                ++q;
+            }
     }
     if (i >= j0 && i < j1) {
         const double d = (double)A[(size_t)i + (size_t)i * n];
         dinv[i] = d != 0 ? 1 / d : 1.0;
     }
-}
-
-__global__ void k_rhs(int n, trsv::GArgs ga, double *g, double *x) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    g[i] = trsv::g_of(ga, i);
-    x[i] = 0;
-}
-
-__global__ void k_apply(int n, const double *x, const double *base, double *out, double *dx) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    dx[i] = x[i];
-    if (out) out[i] = base[i] - x[i];
 }
 
 inline int nb(int n, int t) { return (n + t - 1) / t; }
@@ -339,24 +354,21 @@ void sparse_alloc(Ctx &c) {
     int dev = 0, sms = 0;
     D4_CUDA_OK(cudaGetDevice(&dev));
     D4_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    // about 128 rows per CTA (one row per thread at most): fewer CTAs, cheaper barriers
-    c.sp_grid = std::max(1, std::min(sms, sp::nb(n, 128)));
+    // kRowsPer rows per CTA while the SMs suffice (one row per thread at most): the
+    // barriers cost little more over 128 CTAs than over 32, the SpMV a quarter
+    c.sp_grid = std::max(1, std::min(sms, sp::nb(n, sp::kRowsPer)));
     if (sp::nb(n, c.sp_grid) > sp::kThreads) throw StateError("n too large for the GMRES grid");
     c.sp_nch = sp::nb(n, sp::kChunk);
     auto ialloc = [](int **p, size_t k) { D4_CUDA_OK(d4::dmalloc((void **)p, sizeof(int) * k)); };
     auto dalloc = [](double **p, size_t k) {
         D4_CUDA_OK(d4::dmalloc((void **)p, sizeof(double) * k));
     };
-    ialloc(&c.sp_cnt, (size_t)c.sp_nch * n);
     ialloc(&c.sp_off, (size_t)c.sp_nch * n);
     ialloc(&c.sp_rp, (size_t)n + 1);
-    ialloc(&c.sp_flags, 4);
     D4_CUDA_OK(d4::dmalloc((void **)&c.sp_bar, sizeof(unsigned) * 64));
+    c.sp_flags = (int *)(c.sp_bar + 32);
     dalloc(&c.sp_dinv, n);
-    dalloc(&c.sp_V, (size_t)(sp::kM + 1) * n);
     dalloc(&c.sp_z, n);
-    dalloc(&c.sp_w, n);
-    dalloc(&c.sp_g, n);
     dalloc(&c.sp_x, n);
     dalloc(&c.sp_part, (size_t)2 * c.sp_grid * sp::kStride);
     // initial CSR capacity: 64 entries per row, grown on demand
@@ -366,8 +378,7 @@ void sparse_alloc(Ctx &c) {
 }
 
 void sparse_free(Ctx &c) {
-    void *bufs[] = {c.sp_cnt, c.sp_off, c.sp_rp, c.sp_flags, c.sp_bar, c.sp_dinv, c.sp_V,
-                    c.sp_z, c.sp_w, c.sp_g, c.sp_x, c.sp_part, c.sp_ci, c.sp_val};
+    void *bufs[] = {c.sp_off, c.sp_rp, c.sp_bar, c.sp_dinv, c.sp_z, c.sp_x, c.sp_part, c.sp_ci, c.sp_val};
     for (void *b : bufs)
         if (b) cudaFree(b);
 }
@@ -377,9 +388,10 @@ void sparse_free(Ctx &c) {
 void sparse_prepare(Ctx &c) {
     const int n = c.n;
     const dim3 grid(sp::nb(n, 128), c.sp_nch);
-    sp::k_csr_count<double><<<grid, 128, 0, c.stream>>>(n, c.A, c.sp_cnt);
+    sp::k_csr_count<double><<<sp::nb(n, 32), dim3(32, sp::kCountChunks), 0, c.stream>>>(
+        n, c.sp_nch, c.A, c.sp_off, c.sp_rp);
     check_launch("k_csr_count");
-    sp::k_csr_rows<<<1, 1024, 0, c.stream>>>(n, c.sp_nch, c.sp_cnt, c.sp_off, c.sp_rp);
+    sp::k_csr_rows<<<1, 1024, 0, c.stream>>>(n, c.sp_rp);
     check_launch("k_csr_rows");
     D4_CUDA_OK(cudaMemcpyAsync(c.h_flags, c.sp_rp + n, sizeof(int), cudaMemcpyDeviceToHost,
                                c.stream));
@@ -415,27 +427,28 @@ bool sparse_solve_update(Ctx &c, int gmode, double hval, const double *s_end,
     ga.s_init = s_init;
     ga.x_new = x_new;
     ga.x_old = x_old;
-    sp::k_rhs<<<sp::nb(n, 256), 256, 0, c.stream>>>(n, ga, c.sp_g, c.sp_x);
-    check_launch("k_rhs");
-    D4_CUDA_OK(cudaMemsetAsync(c.sp_bar, 0, sizeof(unsigned) * 64, c.stream));
-    D4_CUDA_OK(cudaMemsetAsync(c.sp_flags, 0, sizeof(int) * 4, c.stream));
+    D4_CUDA_OK(cudaMemsetAsync(c.sp_bar, 0, sizeof(unsigned) * 64, c.stream));  // and sp_flags
     sp::GmresArgs a;
     a.n = n;
     a.rp = c.sp_rp;
     a.ci = c.sp_ci;
     a.val = c.sp_val;
     a.dinv = c.sp_dinv;
-    a.g = c.sp_g;
+    a.g = ga;
+    a.base = base;
+    a.out = out;
+    a.dx = c.dx;
     a.x = c.sp_x;
-    a.V = c.sp_V;
     a.z = c.sp_z;
-    a.w = c.sp_w;
     a.part = c.sp_part;
     a.bar = c.sp_bar;
     a.flags = c.sp_flags;
     void *args[] = {(void *)&a};
+    const size_t smem = sizeof(double) * (sp::kM + 2) * sp::nb(n, c.sp_grid);
+    D4_CUDA_OK(cudaFuncSetAttribute(sp::k_gmres, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)smem));
     D4_CUDA_OK(cudaLaunchCooperativeKernel((const void *)sp::k_gmres, dim3(c.sp_grid),
-                                           dim3(sp::kThreads), args, 0, c.stream));
+                                           dim3(sp::kThreads), args, smem, c.stream));
     check_launch("k_gmres");
     D4_CUDA_OK(cudaMemcpyAsync(c.h_flags, c.sp_flags, sizeof(int) * 4, cudaMemcpyDeviceToHost,
                                c.stream));
@@ -447,8 +460,6 @@ bool sparse_solve_update(Ctx &c, int gmode, double hval, const double *s_end,
         c.sp_fallbacks += 1;
         return false;
     }
-    sp::k_apply<<<sp::nb(n, 256), 256, 0, c.stream>>>(n, c.sp_x, base, out, c.dx);
-    check_launch("k_apply");
     return true;
 }
 
