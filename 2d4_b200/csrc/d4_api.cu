@@ -115,7 +115,7 @@ void free_all(Ctx *c) {
                     c->tol, c->A, c->LU, c->F, c->piv, c->perm, c->flags, c->red,
                     c->wave_err, c->xw1, c->xw2,
                     c->rowsub, c->rowsc,
-                    c->lu_p0, c->lu_q, c->lu_mask, c->lu_bar, c->A32, c->LU32, c->lu32_p0,
+                    c->lu_q, c->lu_mask, c->lu_bar, c->A32, c->LU32, c->lu32_p0,
                     c->lu32_q, c->m_g, c->m_r, c->m_dx, c->m_c32, c->m_w1, c->m_resid,
                     c->m_part, c->m_dx2, c->m_cnt, c->m_conv, c->spiv};
     for (void *b : bufs)
@@ -125,7 +125,7 @@ void free_all(Ctx *c) {
     d4::blu_free(c->m32b.blu);
     if (c->blu_tasks) cudaFree(c->blu_tasks);
     const d4::Mix32Bufs &B = c->m32b;
-    void *ob[] = {c->lub.LU, c->lub.P0, c->lub.Q, c->lub.mask, c->lub.bar, c->lub.perm,
+    void *ob[] = {c->lub.LU, c->lub.Q, c->lub.mask, c->lub.bar, c->lub.perm,
                   c->lub.piv, c->flags3, c->F_b, c->dvec_b, c->speed_b, c->speed2_b, c->xw1_b,
                   c->xw2_b, c->dx_b, B.A32, B.LU32, B.P0, B.Q, B.mask, B.bar, B.perm, B.piv,
                   B.g, B.r, B.dx, B.part, B.c32, B.w1, B.resid, B.dx2, B.cnt, B.conv, B.A64,
@@ -211,8 +211,7 @@ constexpr int kMixedMinN = 2048;
 // Grid split of an attempt's two concurrent cooperative factorisations:
 // stage I's chain (one LU, two solves, one sweep) is the shorter one, so it
 // gets 40% of the co-resident CTAs and stage II's factorisation the rest.
-// Neither gets fewer than one thread per row (n / 256 CTAs), as the full
-// grid's size check requires.
+// Neither gets fewer than one thread per row (n / 256 CTAs).
 static void stage_split(int grid, int n, int &g1, int &g2) {
     const int need = (n + 255) / 256;
     g1 = std::max(need, grid * 2 / 5);
@@ -226,7 +225,7 @@ static void stage_split(int grid, int n, int &g1, int &g2) {
 // stage I's factor buffer the two chains are independent: stage I runs on
 // stream_b with its own factors, force scratch and copies of d and the end
 // speed, while stages II and III run on the context's stream.  The two
-// concurrent cooperative factorisations take half the CTAs each, so both are
+// concurrent cooperative factorisations split the CTAs (stage_split), so both are
 // co-resident; stage III's runs on the full grid.  Every operation is the
 // sequential attempt's, so the results are identical; the factorisations'
 // flags go to separate slots and are read once at the end.
@@ -866,8 +865,8 @@ int d4_create(void **out, int n, const d4_params *p) {
         D4_CUDA_OK(cudaMemset(c->flags, 0, sizeof(int) * d4::kFlagCount));
         c->lu_grid = d4::coop_grid_size(n);
         if (c->lu_grid < 0) throw d4::StateError("n too large for the cooperative LU");
-        dalloc(&c->lu_p0, (size_t)n * 32);
-        dalloc(&c->lu_q, (size_t)n * 128 + d4::kLuDiagWords);
+        dalloc(&c->lu_q, (size_t)n * 160 + d4::kLuDiagWords);
+        c->lu_p0 = c->lu_q + (size_t)n * 128 + d4::kLuDiagWords;
         d4::lu_encode_maps(c->lu_maps, c->LU, c->lu_q + (size_t)n * 64, n);
         c->lu_mask_words = d4::lu_mask_words_for(nblk);
         dalloc(&c->lu_mask, (size_t)c->lu_mask_words);
@@ -904,8 +903,8 @@ int d4_create(void **out, int n, const d4_params *p) {
                 // the FP64 form's stage I (also the mixed form's attempts below
                 // kMixedMinN, which run on the FP64 path)
                 dalloc(&c->lub.LU, nn);
-                dalloc(&c->lub.P0, (size_t)n * 32);
-                dalloc(&c->lub.Q, (size_t)n * 128 + d4::kLuDiagWords);
+                dalloc(&c->lub.Q, (size_t)n * 160 + d4::kLuDiagWords);
+                c->lub.P0 = c->lub.Q + (size_t)n * 128 + d4::kLuDiagWords;
                 dalloc(&c->lub.mask, (size_t)c->lu_mask_words);
                 dalloc(&c->lub.bar, 64);
                 dalloc(&c->lub.perm, (size_t)n);

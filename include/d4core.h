@@ -289,8 +289,8 @@ int d4_pair_tile_threads(void *ctx, int *threads_y);
  * multiplier) and instance k has n[k] dislocations (even, 2..8192, internal
  * order).  Each attempt round runs stages I-IV for every active instance with
  * one launch per phase (all instances' pair tiles and row blocks in one grid;
- * one CTA per instance for an exact-order LU and the substitutions, so each
- * instance reproduces d4_run's arithmetic), then applies each instance's step
+ * one thread-block cluster per instance for the exact-order LU, one CTA for the
+ * substitutions, so each instance reproduces d4_run's arithmetic), then applies each instance's step
  * control as d4_run does (src/simulation.cpp:88-277; no log, sub-configuration
  * or write-out clipping).  An instance stays active until interrupt() holds
  * (time, strain, step-count or avalanche limit, src/simulation.cpp:722-750;
