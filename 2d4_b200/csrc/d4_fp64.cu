@@ -48,14 +48,11 @@ __global__ void k_half_weights64(int n, const double *dvec, double factor, char 
 }
 
 // Elementwise rescale (src/simulation.cpp:584-594): factor of the row.
-__global__ void k_half_rescale64(int n, double *A, const double *fac) {
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t total = (size_t)n * n;
-    if (idx >= total) return;
-    const int r = (int)(idx % n), c = (int)(idx / n);
-    const double f = fac[r];
-    double e = A[idx];
-    A[idx] = (r == c) ? 1 + (e - 1) / 2 * f : e / 2 * f;
+__global__ void __launch_bounds__(kElemThreads) k_half_rescale64(int n, double *A,
+                                                                 const double *fac) {
+    elem_apply(n, A, [=](int r, int c, double e) {
+        return r == c ? 1 + (e - 1) / 2 * fac[r] : e / 2 * fac[r];
+    });
 }
 
 __global__ void k_shift_speed64(int n, double *v, double dif) {
@@ -156,7 +153,7 @@ void jacobian64(Ctx &c, const double *x, const double *y, double h, double ext_a
     if (c.fast_pairs) {
         pairs64_fast(c, true, x, y, c.F, h, c.stream);
         rows64_fast(c, true, c.F, ext_a, ext_b, v_a, v_b, c.stream);
-        k_scale_rows64<<<blocks((long long)c.n * c.n, 256), 256, 0, c.stream>>>(c.n, c.A, c.rowsub,
+        k_scale_rows64<<<elem_grid(c.n), kElemThreads, 0, c.stream>>>(c.n, c.A, c.rowsub,
                                                                                c.rowsc);
         check_launch("k_scale_rows64");
         return;
@@ -182,7 +179,7 @@ void jacobian64(Ctx &c, const double *x, const double *y, double h, double ext_a
     r.wfn = c.p.weight_function;
     r.err = c.wave_err + kWaveErrRows;
     launch_rows<true>(c, r, c.stream);
-    k_scale_rows64<<<blocks((long long)c.n * c.n, 256), 256, 0, c.stream>>>(c.n, c.A, c.rowsub,
+    k_scale_rows64<<<elem_grid(c.n), kElemThreads, 0, c.stream>>>(c.n, c.A, c.rowsub,
                                                                            c.rowsc);
     check_launch("k_scale_rows64");
 }
@@ -251,7 +248,7 @@ void jacobian_from_prev64(Ctx &c, double factor) {
                                                              c.p.weight_function, c.dvec_new,
                                                              c.fac);
     check_launch("k_half_weights64");
-    k_half_rescale64<<<blocks((long long)c.n * c.n, 256), 256, 0, c.stream>>>(c.n, c.A, c.fac);
+    k_half_rescale64<<<elem_grid(c.n), kElemThreads, 0, c.stream>>>(c.n, c.A, c.fac);
     check_launch("k_half_rescale64");
     D4_CUDA_OK(cudaMemcpyAsync(c.dvec, c.dvec_new, sizeof(double) * c.n, cudaMemcpyDeviceToDevice,
                                c.stream));

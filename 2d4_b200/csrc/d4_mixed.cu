@@ -34,13 +34,22 @@ namespace {
 
 // FP64 matrix -> FP32, rows gathered through perm (null: identity):
 // A32[r + c n] = A[perm[r] + c n].
-__global__ void k_to32(int n, const double *__restrict__ A, const int *__restrict__ perm,
-                       float *__restrict__ A32) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    const int c = blockIdx.y;
+// Bound by the memory: kTo32Cols columns per thread, their loads first (n = 4096:
+// 31 us for 201 MB; 52 with one entry per thread).
+constexpr int kTo32Cols = 8;
+__global__ void __launch_bounds__(256) k_to32(int n, const double *__restrict__ A,
+                                              const int *__restrict__ perm,
+                                              float *__restrict__ A32) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x, c0 = blockIdx.y * kTo32Cols;
     if (r >= n) return;
-    const int src = perm ? perm[r] : r;
-    A32[(size_t)r + (size_t)c * n] = (float)A[(size_t)src + (size_t)c * n];
+    const double *src = A + (perm ? perm[r] : r) + (size_t)c0 * n;
+    double v[kTo32Cols];
+#pragma unroll
+    for (int u = 0; u < kTo32Cols; ++u)
+        if (c0 + u < n) v[u] = src[(size_t)u * n];
+#pragma unroll
+    for (int u = 0; u < kTo32Cols; ++u)
+        if (c0 + u < n) A32[(size_t)r + (size_t)(c0 + u) * n] = (float)v[u];
 }
 
 __device__ __forceinline__ unsigned long long obits(double v) {
@@ -257,13 +266,13 @@ void factor32_async(Ctx &c, const Mix32Bufs &B, const double *A, bool copy_matri
     *B.blk = c.m_fast;
     if (c.m_fast) {
         // block LU (d4_blu32.cu) of the row-permuted FP32 matrix
-        k_to32<<<dim3(nb(n, 256), n), 256, 0, st>>>(n, src, c.spiv, B.A32);
+        k_to32<<<dim3(nb(n, 256), nb(n, kTo32Cols)), 256, 0, st>>>(n, src, c.spiv, B.A32);
         check_launch("k_to32");
         blu_factor_async(B.blu, n, B.A32, B.LU32, B.flags, grid, st);
         ++c.m_blocklu;
         return;
     }
-    k_to32<<<dim3(nb(n, 256), n), 256, 0, st>>>(n, src, nullptr, B.LU32);
+    k_to32<<<dim3(nb(n, 256), nb(n, kTo32Cols)), 256, 0, st>>>(n, src, nullptr, B.LU32);
     check_launch("k_to32");
     D4_CUDA_OK(cudaMemsetAsync(B.bar, 0, sizeof(unsigned) * 64, st));
     D4_CUDA_OK(cudaMemsetAsync(B.mask, 0, sizeof(unsigned) * c.lu_mask_words, st));
