@@ -202,7 +202,7 @@ __global__ void k_ens_half_finish(Pools P, const Inst *ins, const Sc *sc, const 
 // instance.  The cluster takes the place of the grid of the single-system LU:
 // its barriers are the hardware's, and a large instance's LU is spread over
 // several SMs (one CTA per instance took 168 ms for n = 2048, the length of the
-// whole round's factorisation; a cluster of 4 takes 20 ms).
+// whole round's factorisation; a cluster of 4 takes 17.6 ms).
 __global__ void __launch_bounds__(lux::kThreads, 1) k_ens_lu(Pools P, const Inst *ins,
                                                              const int *act) {
     lux::ClusterGroup g;
@@ -449,7 +449,7 @@ void autotune(Ensemble &E) {
 // CTAs per instance of the LU: the smallest power of two that keeps the largest
 // active instance's factorisation within the others' share of the chip,
 // n_max^3 / G <= sum n^3 / SMs (the work is n^3, and a cluster's efficiency
-// hardly depends on its size: n = 1024 takes 11.7, 6.7, 3.2 and 1.7 ms on 1, 2, 4
+// hardly depends on its size: n = 1024 takes 9.3, 6.0, 2.8 and 1.5 ms on 1, 2, 4
 // and 8 CTAs), at most 8 (the portable size).
 int lu_cluster(const Ensemble &E) {
     double sum = 0, top = 0;

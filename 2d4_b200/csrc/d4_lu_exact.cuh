@@ -35,10 +35,11 @@
 // The next block's pass waits for that publication and those tiles only, so a
 // block without swaps costs one group barrier.  Every wait is bounded.
 //
-// What bounds it.  At N <= 1024 the chain of one block: diagonal elimination
-// (an FP64 division of 125 cycles, a product, a difference and a CTA barrier
-// per column), publication, rows below (a 5-operation quotient per column),
-// group barrier (2400 cycles over a grid).  At N = 4096 the update, at the
+// What bounds it.  At N <= 1024 the look-ahead's chain of one block, 26,500 cycles:
+// its 32 rows and columns 5,500, their update 1,900, the elimination 8,800 (a
+// reciprocal, a quotient, a product and a difference per column), loads, verdict and
+// publication the rest; the others' chain (their rows and columns, the group
+// barrier's 2,400, the strips) is 7,000 shorter.  At N = 4096 the update, at the
 // rate of separate FP64 products and differences (64 lanes per clock and SM).
 // One CTA of 256 threads per SM: the chains and the 8 x 4 update tiles need
 // more than the 128 registers that 512 threads leave.
