@@ -65,9 +65,12 @@ constexpr long long kSpinLimit = 1ll << 25;  // polls: > 1 s
 // backward: k descending, then the division), so the result equals the
 // sequential substitution's.  (The oracle skips updates with a zero value; here
 // they are applied: x - l*0 == x.)  Waits are bounded: after kSpinLimit polls a
-// warp records err[0] and stops waiting (the host then discards the results);
-// all CTAs meet at a final cluster barrier, so none exits while another may
-// still write into its shared memory.
+// warp records err[0] and stops waiting (the host then discards the results).
+// Before the final cluster barrier every CTA waits for all groups of its own
+// copy of x.  An asynchronous store is complete only when its mbarrier says so (no
+// CTA or cluster barrier orders it), and nobody has waited for the block solved
+// last, whose values no other block applies: without this wait a CTA could exit,
+// or a second pass set its barriers up again, with stores still on their way.
 constexpr int kClusterCtas = 8;
 constexpr int kClusterMaxWarps = 8;
 
@@ -330,11 +333,26 @@ __device__ __forceinline__ void solve_pass(int n, const T *__restrict__ LU,
         }
     }
     __syncthreads();
+    bool gave_up = false;
+    for (int b = tid; b * 8 < n; b += blockDim.x) {
+        const uint32_t ma = static_cast<uint32_t>(__cvta_generic_to_shared(mbar + b));
+        long long spins = 0;
+        while (!gave_up && !try_wait_cluster(ma))
+            if (++spins > kSpinLimit) {
+                gave_up = true;
+                if (atomicCAS(err, 0, 1) == 0) {
+                    err[1] = -1;
+                    err[2] = b >> 2;
+                    err[3] = -1;
+                    err[4] = -1;
+                }
+            }
+    }
     cluster_sync_all();
 }
 
-// Between two passes of one launch by a lone CTA: frees the first pass's
-// barriers, so that the second can set them up again.
+// Between two passes of one launch by a lone CTA (all stores of the first pass have
+// landed, see above): frees its barriers, so that the second can set them up again.
 __device__ __forceinline__ void release_barriers(int n, size_t elem) {
     extern __shared__ __align__(16) unsigned char craw[];
     uint64_t *mbar = reinterpret_cast<uint64_t *>(craw + ((elem * (size_t)n + 15) / 16) * 16);
