@@ -650,8 +650,10 @@ int d4_ensemble_create(void **out, int count, const int *n, const d4_params *p) 
         E->solve_smem = (int)d4::trsv::cluster_smem_bytes<double>((int)smax);
         D4_CUDA_OK(cudaFuncSetAttribute(k_ens_lu, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)sizeof(d4::lux::Smem)));
+        // the largest size's, as the limit is the process's: an ensemble created later,
+        // of smaller instances, must not lower it
         D4_CUDA_OK(cudaFuncSetAttribute(k_ens_solve, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        E->solve_smem));
+                                        (int)d4::trsv::cluster_smem_bytes<double>(d4::kMaxSolveN)));
         D4_CUDA_OK(cudaFuncSetAttribute(k_ens_rows<true>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         d4::row_smem_bytes<true>()));
