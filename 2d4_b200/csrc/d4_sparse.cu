@@ -39,6 +39,9 @@ constexpr int kRowsPer = 32;      // rows per CTA as long as the SMs suffice
 constexpr long long kSpinLimit = 1ll << 22;  // polls of several hundred cycles: > 1 s
 constexpr double kTol = 1e-13;
 
+// The basis and w of the rows of a CTA.
+constexpr size_t gmres_smem_bytes(int rows) { return sizeof(double) * (kM + 2) * rows; }
+
 struct GmresArgs {
     int n;
     const int *rp, *ci;
@@ -358,6 +361,10 @@ void sparse_alloc(Ctx &c) {
     // barriers cost little more over 128 CTAs than over 32, the SpMV a quarter
     c.sp_grid = std::max(1, std::min(sms, sp::nb(n, sp::kRowsPer)));
     if (sp::nb(n, c.sp_grid) > sp::kThreads) throw StateError("n too large for the GMRES grid");
+    // for any number of rows per CTA: the limit is the process's, and other contexts
+    // launch from other threads
+    D4_CUDA_OK(cudaFuncSetAttribute(sp::k_gmres, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)sp::gmres_smem_bytes(sp::kThreads)));
     c.sp_nch = sp::nb(n, sp::kChunk);
     auto ialloc = [](int **p, size_t k) { D4_CUDA_OK(d4::dmalloc((void **)p, sizeof(int) * k)); };
     auto dalloc = [](double **p, size_t k) {
@@ -444,9 +451,7 @@ bool sparse_solve_update(Ctx &c, int gmode, double hval, const double *s_end,
     a.bar = c.sp_bar;
     a.flags = c.sp_flags;
     void *args[] = {(void *)&a};
-    const size_t smem = sizeof(double) * (sp::kM + 2) * sp::nb(n, c.sp_grid);
-    D4_CUDA_OK(cudaFuncSetAttribute(sp::k_gmres, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem));
+    const size_t smem = sp::gmres_smem_bytes(sp::nb(n, c.sp_grid));
     D4_CUDA_OK(cudaLaunchCooperativeKernel((const void *)sp::k_gmres, dim3(c.sp_grid),
                                            dim3(sp::kThreads), args, smem, c.stream));
     check_launch("k_gmres");

@@ -27,3 +27,31 @@ def test_small_ensemble_beside_a_large_one(pkg):
     assert np.array_equal(large.positions(0)[0], want)
     small.close()
     large.close()
+
+def test_gmres_contexts_on_two_threads(pkg):
+    """Two contexts whose GMRES takes different numbers of rows per CTA (20 and 32)."""
+    import threading
+
+    errors = []
+
+    def steps(n):
+        x, y, _ = pkg.dconf.generate_internal(n, n)
+        sd = pkg.SimulationData()
+        sd.set_positions(x, y)
+        sd.cutoff_multiplier, sd.heaviside_cutoff = 3.2, True
+        sd.solver = pkg._lib.D4_SOLVER_GMRES
+        e = pkg.Engine(sd)
+        try:
+            want = e.attempt(0.0, 1e-5)[1]
+            for _ in range(400):
+                assert np.array_equal(e.attempt(0.0, 1e-5)[1], want)
+        except Exception as err:
+            errors.append((n, err))
+        e.close()
+
+    threads = [threading.Thread(target=steps, args=(n,)) for n in (40, 64)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
