@@ -336,11 +336,11 @@ void rows64_fast(Ctx &c, bool jac, const double *F, double ext_a, double ext_b, 
 void speeds64_with(Ctx &c, double *F, cudaStream_t st, const double *x, const double *y,
                    double ext, double *v);
 // Plain solve of A dx = g (g on device, dx written to c.dx).
-void solve_plain64(Ctx &c, const double *g);
+void solve_plain64(Ctx &c, const double *g, bool skip = false);
 // Mixed form: refined solve of A32 dx = g with the last factorisation (g on
 // device, dx written to c.dx); the block LU's factorisation falls back to the
 // pivoted one by itself when a diagonal tile met a bad pivot (factor32).
-void solve_plain32(Ctx &c, const double *g);
+void solve_plain32(Ctx &c, const double *g, bool skip = false);
 
 // ---- mixed form (d4_mixed.cu) ----
 // Refinement sweeps: at most kIrMax, stopping once max|r| <= kIrStop max|g|.

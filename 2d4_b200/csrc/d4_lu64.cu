@@ -15,9 +15,10 @@
 namespace d4 {
 using trsv::GArgs;
 
+template <bool kSkip = false>
 static void launch_solve(Ctx &c, const GArgs &ga) {
-    trsv::launch_cluster_solve<double>(c.n, c.LU, c.perm, c.flags, ga, c.xw1, c.xw2, c.wave_err,
-                                       c.stream);
+    trsv::launch_cluster_solve<double, false, kSkip>(c.n, c.LU, c.perm, c.flags, ga, c.xw1, c.xw2,
+                                                     c.wave_err, c.stream);
 }
 
 void solve_update64(Ctx &c, int gmode, double hval, const double *s_end, const double *s_init,
@@ -57,12 +58,15 @@ void solve_update64_with(Ctx &c, const LuBufs &L, const SolveBufs &S, cudaStream
                                        st);
 }
 
-void solve_plain64(Ctx &c, const double *g) {
+void solve_plain64(Ctx &c, const double *g, bool skip) {
     GArgs ga{};
     ga.gmode = -1;
     ga.g_in = g;
     ga.dx_out = c.dx;
-    launch_solve(c, ga);
+    if (skip)
+        launch_solve<true>(c, ga);
+    else
+        launch_solve(c, ga);
 }
 
 }  // namespace d4

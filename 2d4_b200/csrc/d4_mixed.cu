@@ -344,11 +344,11 @@ int coop_grid_size32(int n) {
 
 // FP32 solve with B's factors: LU32^-1 r (r FP64 in, result FP32), by the
 // block solves of the block LU (rows of r through the static pivots), or by
-// the cluster solve of the pivoted LU.  Sweep `it` of the refinement: the
-// block solve returns at once when sweep it - 1 converged.  Returns the
-// result's buffer.
+// the cluster solve of the pivoted LU (`skip`: its kSkip form).  Sweep `it` of the
+// refinement: the block solve returns at once when sweep it - 1 converged.
+// Returns the result's buffer.
 static const float *solve32_once(Ctx &c, const Mix32Bufs &B, cudaStream_t st, const double *r,
-                                 int it) {
+                                 int it, bool skip) {
     if (*B.blk) {
         blu_solve_async(B.blu, c.n, B.LU32, r, c.spiv, B.conv, it, B.flags, st);
         return B.blu.xs;
@@ -356,8 +356,9 @@ static const float *solve32_once(Ctx &c, const Mix32Bufs &B, cudaStream_t st, co
     trsv::GArgs g{};
     g.gmode = -1;
     g.g_in = r;
-    trsv::launch_cluster_solve<float>(c.n, B.LU32, B.perm, B.flags, g, B.w1, B.c32, c.wave_err,
-                                      st);
+    const auto solve = skip ? trsv::launch_cluster_solve<float, false, true>
+                            : trsv::launch_cluster_solve<float, false, false>;
+    solve(c.n, B.LU32, B.perm, B.flags, g, B.w1, B.c32, c.wave_err, st);
     return B.c32;
 }
 
@@ -365,11 +366,11 @@ static const float *solve32_once(Ctx &c, const Mix32Bufs &B, cudaStream_t st, co
 // c = LU32^-1 r, dx += c, r = g - A dx, until converged or kIrMax sweeps; dx
 // alternates between B.dx and B.dx2, and a converged sweep only carries it
 // over, so after kIrMax launches the buffer is known on the host.  Returns it.
-static const double *refine(Ctx &c, const Mix32Bufs &B, cudaStream_t st) {
+static const double *refine(Ctx &c, const Mix32Bufs &B, cudaStream_t st, bool skip = false) {
     const int n = c.n, nch = nb(n, kResidCols);
     double *dxa = B.dx, *dxb = B.dx2;
     for (int it = 0; it < kIrMax; ++it) {
-        const float *corr = solve32_once(c, B, st, B.r, it);
+        const float *corr = solve32_once(c, B, st, B.r, it, skip);
         k_resid_fused<<<dim3(nb(n, kResidRows), nch), kResidThreads, 0, st>>>(
             n, B.A64, dxa, corr, dxb, B.g, B.part, nch, B.cnt, B.r, B.conv, it);
         check_launch("k_resid_fused");
@@ -407,14 +408,14 @@ void solve_update32_with(Ctx &c, const Mix32Bufs &B, const double *dvec, double 
     check_launch("k_ir_apply");
 }
 
-void solve_plain32(Ctx &c, const double *g) {
+void solve_plain32(Ctx &c, const double *g, bool skip) {
     const int n = c.n;
     Mix32Bufs B = primary_mix32(c);
     trsv::GArgs ga{};
     ga.gmode = -1;
     ga.g_in = g;
     ir_start(c, B, c.stream, ga);
-    const double *dx = refine(c, B, c.stream);
+    const double *dx = refine(c, B, c.stream, skip);
     k_absmax2<<<64, 256, 0, c.stream>>>(n, B.r, B.g, B.resid + 2 * *B.resid_count);
     check_launch("k_absmax2");
     *B.resid_count = (*B.resid_count + 1) % 8;
