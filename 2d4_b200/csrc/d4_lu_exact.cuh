@@ -392,7 +392,9 @@ __device__ __forceinline__ unsigned eliminate(double (&c)[4], bool &bad) {
 }
 
 // The same elimination with IEEE divisions, for blocks with values outside the
-// quotient window or zero pivots, and for passes that skip singular columns.
+// quotient window or zero pivots, and for passes that skip singular columns.  Its
+// multipliers may be infinite or NaN, so it skips updates by a zero as the oracle does
+// (and so do row_below_slow and col_slow).
 // All threads call it (warps 0..7 pass their columns, the others idle).
 static __device__ __noinline__ unsigned eliminate_slow(const double (&c0)[4], int kw,
                                                 unsigned skip) {
@@ -425,7 +427,7 @@ static __device__ __noinline__ unsigned eliminate_slow(const double (&c0)[4], in
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const double u = __shfl_sync(0xffffffffu, c[j], k);
-                if (lane > k && 4 * w + j > k) c[j] = c[j] - l * u;
+                if (lane > k && 4 * w + j > k && u != 0.0) c[j] = c[j] - l * u;
             }
         }
     }
@@ -517,11 +519,13 @@ static __device__ __noinline__ unsigned row_below_slow(const Args &a, double *Q,
             if ((skip >> k) & 1u) continue;
             const double d = S.s[k][k];
             if (fabs(v) > fabs(d)) msk |= 1u << k;
-            const double l = v / d;
-            const double cs = c[s] - l * S.s[k][q + kLanes * s];
-            c[s] = q == own ? l : (q > own ? cs : c[s]);
+            const double l = v / d, us = S.s[k][q + kLanes * s];
+            c[s] = q == own ? l : (q > own && us != 0.0 ? c[s] - l * us : c[s]);
 #pragma unroll
-            for (int t = s + 1; t < kHold; ++t) c[t] = c[t] - l * S.s[k][q + kLanes * t];
+            for (int t = s + 1; t < kHold; ++t) {
+                const double u = S.s[k][q + kLanes * t];
+                if (u != 0.0) c[t] = c[t] - l * u;
+            }
         }
     }
     if (active) row_store(a, Q, r_pos, k0, pre, c);
@@ -560,7 +564,8 @@ __device__ __forceinline__ bool row_core(double (&c)[kHold], double (&pre)[kHold
 
 // U12 of one column, kLanes lanes per column: lane q holds rows q, q + kLanes,
 // ...; the next row's value is formed from a broadcast a step early, as above.
-__device__ __forceinline__ void col_core(double (&c)[kHold]) {
+// False when some value is not finite: col_slow then solves the column.
+__device__ __forceinline__ bool col_core(double (&c)[kHold]) {
     Smem &S = smem();
     const int lane = threadIdx.x & 31, q = lane % kLanes, gb = lane - q;
     double u = __shfl_sync(0xffffffffu, c[0], gb);
@@ -577,6 +582,36 @@ __device__ __forceinline__ void col_core(double (&c)[kHold]) {
             for (int t = s + 1; t < kHold; ++t) c[t] = c[t] - S.s[q + kLanes * t][k] * u;
             u = un - S.s[k < 31 ? k + 1 : 31][k] * u;
         }
+    }
+    bool good = true;
+#pragma unroll
+    for (int t = 0; t < kHold; ++t) good = good && isfinite(c[t]);
+    return __all_sync(0xffffffffu, good);
+}
+static __device__ __noinline__ void col_slow(const Args &a, double *U, int pos, int k0,
+                                             bool active) {
+    Smem &S = smem();
+    const int lane = threadIdx.x & 31, q = lane % kLanes, gb = lane - q;
+    double c[kHold];
+#pragma unroll
+    for (int t = 0; t < kHold; ++t)
+        c[t] = active ? a.A[(size_t)(k0 + q + kLanes * t) + (size_t)pos * a.n] : 0.0;
+#pragma unroll
+    for (int s = 0; s < kHold; ++s) {
+#pragma unroll 1
+        for (int own = 0; own < kLanes; ++own) {
+            const int k = kLanes * s + own;
+            const double u = __shfl_sync(0xffffffffu, c[s], gb + own);
+            if (u != 0.0) {
+                if (q > own) c[s] = c[s] - S.s[q + kLanes * s][k] * u;
+#pragma unroll
+                for (int t = s + 1; t < kHold; ++t) c[t] = c[t] - S.s[q + kLanes * t][k] * u;
+            }
+        }
+    }
+    if (active) {
+#pragma unroll
+        for (int t = 0; t < kHold; ++t) U[(size_t)(q + kLanes * t) * a.n + pos] = c[t];
     }
 }
 
@@ -1016,7 +1051,11 @@ __device__ __forceinline__ void factor(const Args &a, Group g) {
                         row_store(a, Q, pos, k0, pre, c);
                     }
                 } else {
-                    col_core(c);
+                    good = col_core(c);
+                    if (!good && !spec) {
+                        col_slow(a, U, pos, k0, active);
+                        continue;
+                    }
                     double *dst = spec ? Up + q * NB + m : U + (size_t)q * n + pos;
                     const size_t step = spec ? kLanes * NB : (size_t)kLanes * n;
                     if (active || spec) {

@@ -54,3 +54,17 @@ def test_overflowed_column_mixed(pkg):
     dx, _ = e.solve(np.ones(n))
     assert np.isfinite(dx).all()
     e.close()
+
+
+@pytest.mark.parametrize("n,row,col", [(32, 5, 2), (32, 31, 30), (66, 5, 2), (130, 63, 40)])
+def test_nan_multiplier_of_zeros(pkg, restated, n, row, col):
+    """A NaN multiplier whose row of U, and whose unknown, are zeros: no effect in the
+    block's own rows and in the columns right of it."""
+    a = np.eye(n) + np.triu(np.full((n, n), 0.25), 1)
+    a[col, col + 1:] = 0
+    a[row, col] = np.nan
+    g = np.random.default_rng(n).normal(size=n)
+    g[col] = 0
+    want = restated.lu_solve(a, g)[0]
+    assert np.isfinite(want).all()
+    assert np.array_equal(factor_solve(pkg, a, [g])[0], want)
