@@ -1519,13 +1519,14 @@ long long d4_device_allocations(void) { return d4::g_allocs.load(); }
 
 int d4_wait_selftest(void *ctx, int which) {
     Ctx *c = (Ctx *)ctx;
-    if (!c || which < 0 || which > 1) return D4_ERR_ARG;
+    if (!c || which < 0 || which > 2) return D4_ERR_ARG;
     D4_GUARD_BEGIN
     D4_CUDA_OK(cudaSetDevice(c->p.device));
     const int st = d4::wait_selftest(which);
     if (st == D4_ERR_STATE)
-        return fail(c, st, which == 0 ? "grid barrier wait gave up (self-test)"
-                                      : "tile flag wait gave up (self-test)");
+        return fail(c, st, which == 0   ? "grid barrier wait gave up (self-test)"
+                           : which == 1 ? "tile flag wait gave up (self-test)"
+                                        : "elimination wait gave up (self-test)");
     return st;
     D4_GUARD_END(c)
 }

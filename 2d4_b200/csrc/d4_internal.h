@@ -381,6 +381,7 @@ void blu_factor_async(const BluBufs &B, int n, const float *A, float *LU, int *f
                       cudaStream_t st);
 // Runs a bounded wait on a barrier or flag that nothing completes (d4_wait_selftest).
 int wait_selftest(int which);
+void elim_wait_selftest(int *flags);  // which = 2 (d4_lu_coop64.cu)
 // x = (block LU of P A)^-1 P b in FP32 (b FP64; perm: the rows of P, null for
 // the identity); the result is B.xs (padded to 128-row blocks).  Refinement
 // sweep `it`: returns at once when conv says sweep it - 1 converged.

@@ -14,7 +14,33 @@ __global__ void __launch_bounds__(kThreads, 1)
     factor(a, GridGroup{bar, 0u, 0u, false});
 }
 
+// Self-test: an elimination whose columns' barriers lack an arrival.
+__global__ void __launch_bounds__(kThreads, 1) k_elim_wait_selftest(int *flags) {
+    Smem &S = smem();
+    if (threadIdx.x == 0) {
+        S.dead = 0;
+        S.stuck = 0;
+        S.parity = 0;
+    }
+    if (threadIdx.x < NB) bulk::init(&S.done[threadIdx.x], 2);
+    bulk::fence_init();
+    __syncthreads();
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double c[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c[i] = lane == 4 * w + i ? 2.0 : 0.01;
+    eliminate_any(c, NB, 0u, flags);
+}
+
 }  // namespace lux
+
+void elim_wait_selftest(int *flags) {
+    const int bytes = (int)sizeof(lux::Smem);
+    D4_CUDA_OK(cudaFuncSetAttribute(lux::k_elim_wait_selftest,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    lux::k_elim_wait_selftest<<<1, lux::kThreads, bytes>>>(flags);
+    check_launch("k_elim_wait_selftest");
+}
 
 // Tensor maps of a factorisation's buffers: A (n x n, column-major) and the two
 // U12 halves (64 rows of n).

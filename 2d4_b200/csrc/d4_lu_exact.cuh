@@ -101,6 +101,7 @@ struct Smem {
     unsigned cta_mask;
     int ns;
     int dead;                       // a bounded wait gave up: stop waiting
+    int stuck;                      // a wait of the elimination gave up
     unsigned parity;                // phase of the mbarriers' next elimination
     unsigned verdict;               // the pass's flagged columns, after the group barrier
     unsigned la_mask;               // look-ahead: flags of the published diagonal block
@@ -296,10 +297,12 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
 __device__ __forceinline__ void mbar_arrive(uint64_t *b) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(b)) : "memory");
 }
-__device__ __forceinline__ void mbar_wait(uint64_t *b, uint32_t parity) {
-    // the arrival is an earlier warp's of this CTA; bounded like every wait
-    for (long long k = 0; k < kSpinLimit; ++k) {
-        uint32_t done;
+// 0 when the wait gave up.  (The arrival is an earlier warp's of this CTA, within
+// microseconds; a poll takes 1.5 us.  An elimination may run into 28 such waits, so
+// their limit is short.)
+__device__ __forceinline__ uint32_t mbar_wait(uint64_t *b, uint32_t parity) {
+    uint32_t done = 0;
+    for (long long k = 0; k < (1 << 16) && !done; ++k) {
         asm volatile(
             "{\n\t.reg .pred P1;\n\t"
             "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
@@ -307,8 +310,8 @@ __device__ __forceinline__ void mbar_wait(uint64_t *b, uint32_t parity) {
             : "=r"(done)
             : "r"(smem_u32(b)), "r"(parity)
             : "memory");
-        if (done) return;
     }
+    return done;
 }
 
 // Eliminates the 32 x 32 diagonal block without pivoting by warps 0..7: warp w
@@ -324,13 +327,14 @@ __device__ __forceinline__ void mbar_wait(uint64_t *b, uint32_t parity) {
 // >= kw) are those of an identity.  Returns the thread's flags: columns where a
 // row has |a_ik| > |a_kk|, which for correctly rounded quotients is |l| > 1.
 // `bad`: some quotient is outside the window; the caller redoes the block with
-// eliminate_slow.  Writes S.s, S.q, S.rs.
+// eliminate_slow.  Writes S.s, S.q, S.rs; S.stuck when a wait gives up.
 __device__ __forceinline__ unsigned eliminate(double (&c)[4], bool &bad) {
     Smem &S = smem();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t par = S.parity;
     unsigned msk = 0;
     bool good = true;
+    uint32_t arrived = 1;
 #pragma unroll 1
     for (int o = 0; o < w; ++o) {
 #pragma unroll
@@ -339,7 +343,7 @@ __device__ __forceinline__ unsigned eliminate(double (&c)[4], bool &bad) {
             double u[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) u[j] = __shfl_sync(0xffffffffu, c[j], k);
-            mbar_wait(&S.done[k], par);
+            arrived &= mbar_wait(&S.done[k], par);
             const double l = S.lcol[k][lane];  // 0 for rows <= k
 #pragma unroll
             for (int j = 0; j < 4; ++j) c[j] = c[j] - l * u[j];
@@ -387,6 +391,7 @@ __device__ __forceinline__ unsigned eliminate(double (&c)[4], bool &bad) {
         good = good && recip_ok(piv[i], e2s[i]) && (!low || value_ok(pre[i]));
         if (low && fabs(c[i]) > 1.0) msk |= 1u << (k0 + i);
     }
+    if (!arrived) S.stuck = 1;
     bad = !good;
     return msk;
 }
@@ -437,17 +442,25 @@ static __device__ __noinline__ unsigned eliminate_slow(const double (&c0)[4], in
 }
 
 // Eliminates c by the fast path, or the slow one where that has to be; all
-// threads call it.  Afterwards S.s, S.q and S.rs are complete.
+// threads call it.  Afterwards S.s, S.q and S.rs are complete.  A wait that gave up
+// is recorded in flags, and the CTA's later eliminations take the slow path, which has
+// no such waits.
 static __device__ __noinline__ unsigned eliminate_any(const double (&c0)[4], int kw,
-                                                  unsigned skip) {
+                                                  unsigned skip, int *flags) {
     Smem &S = smem();
     unsigned msk = 0;
-    bool bad = false;
-    if (skip == 0) {
+    bool bad = S.dead != 0;
+    if (skip == 0 && !bad) {
         double c[4] = {c0[0], c0[1], c0[2], c0[3]};
         msk = eliminate(c, bad);
         bad = __syncthreads_or(bad);
-        if (threadIdx.x == 0) S.parity ^= 1u;
+        if (threadIdx.x == 0) {
+            S.parity ^= 1u;
+            if (S.stuck) {
+                atomicOr(&flags[kFlagBarrierTimeout], 1);
+                S.dead = 1;
+            }
+        }
     }
     if (skip != 0 || bad) msk = eliminate_slow(c0, kw, skip);
     __syncthreads();
@@ -470,7 +483,7 @@ static __device__ __noinline__ unsigned diag_from_p0(const Args &a, double *Q, i
             c[i] = (ok && k < kw) ? a.P0[(size_t)sr * NB + k] : (lane == k ? 1.0 : 0.0);
         }
     }
-    const unsigned msk = eliminate_any(c, kw, skip);
+    const unsigned msk = eliminate_any(c, kw, skip, a.flags);
     if (write_q)
         for (int t = tid; t < NB * NB; t += kThreads) {
             const int r = t / NB, k = t % NB;
@@ -652,7 +665,7 @@ struct Tiling {
 // ([k][row], [k][column]): the 32 updates in the order of the tile that owns
 // it, then its elimination.  Leaves the updated entries in c.
 __device__ __forceinline__ void next_diag(double (&c)[4], const double *Lp,
-                                          const double *Up, int nkw) {
+                                          const double *Up, int nkw, int *flags) {
     Smem &S = smem();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (w < 8) {
@@ -676,7 +689,7 @@ __device__ __forceinline__ void next_diag(double (&c)[4], const double *Lp,
         }
     }
     if (threadIdx.x == 0) S.la_mask = 0;
-    const unsigned m = eliminate_any(c, nkw, 0u);
+    const unsigned m = eliminate_any(c, nkw, 0u, flags);
     if (m) atomicOr(&S.la_mask, m);
 }
 
@@ -729,7 +742,7 @@ static __device__ __noinline__ void look_ahead(const Args &a, int k0, int kb, in
         }
     }
     __syncthreads();
-    next_diag(c, Lp, Up, nkw);
+    next_diag(c, Lp, Up, nkw, a.flags);
     publish(a, c, nk0, nkw, kb, pass);
 }
 
@@ -904,6 +917,7 @@ __device__ __forceinline__ void factor(const Args &a, Group g) {
     const int nblk = (n + NB - 1) / NB;
     if (tid == 0) {
         S.dead = 0;
+        S.stuck = 0;
         S.parity = 0;
     }
     if (tid < NB)
@@ -1066,7 +1080,7 @@ __device__ __forceinline__ void factor(const Args &a, Group g) {
             }
             if (spec) {
                 early = __syncthreads_and(good);
-                if (early) next_diag(c_next, Lp, Up, min(NB, rest));
+                if (early) next_diag(c_next, Lp, Up, min(NB, rest), a.flags);
             } else {
                 if (my_mask) atomicOr(&S.cta_mask, my_mask);
                 fence_bulk();

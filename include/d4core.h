@@ -370,9 +370,11 @@ long long d4_kernel_launches(void);
 /* Self-test of the kernels' bounded waits (no counterpart in the reference):
  * which = 0 runs the cooperative LU's grid barrier with one CTA that never
  * arrives, which = 1 the block LU's tile-flag wait on a flag that nothing
- * sets.  The wait gives up after its normal limit (about a second), the
- * kernel records the timeout and returns, and the call returns D4_ERR_STATE
- * (D4_OK would mean the wait did not give up); the context stays usable. */
+ * sets, which = 2 the FP64 LU's elimination of a diagonal block with column
+ * barriers that lack an arrival.  The wait gives up after its normal limit (about a
+ * second; which = 2 runs into several in turn), the kernel records the timeout and
+ * returns, and the call returns D4_ERR_STATE (D4_OK would mean the wait did not
+ * give up); the context stays usable. */
 int d4_wait_selftest(void *ctx, int which);
 
 /* Number of device allocations (cudaMalloc) this library has made in the
