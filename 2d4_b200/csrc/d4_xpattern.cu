@@ -207,28 +207,31 @@ __global__ void __launch_bounds__(128) k_xp_sum(int K, int slices, const double2
 // a larger size, a failed allocation of the library or the process's end frees it.
 class Spare {
   public:
-    cudaError_t take(char **p, size_t bytes) {
+    // *size: the block's own size, at least `bytes`; give gets it back.
+    cudaError_t take(char **p, size_t bytes, size_t *size) {
         int dev = -1;
         cudaGetDevice(&dev);
         {
             std::lock_guard<std::mutex> lock(m_);
             if (p_ && dev_ == dev && size_ >= bytes) {
                 *p = p_;
+                *size = size_;
                 p_ = nullptr;
                 return cudaSuccess;
             }
         }
         release();
+        *size = bytes;
         return dmalloc(p, bytes);
     }
-    void give(char *p, size_t bytes, bool keep) {
+    void give(char *p, size_t size, bool keep) {
         int dev = -1;
         if (!p) return;
-        if (keep && bytes <= kKeep && cudaGetDevice(&dev) == cudaSuccess) {
+        if (keep && size <= kKeep && cudaGetDevice(&dev) == cudaSuccess) {
             std::lock_guard<std::mutex> lock(m_);
             if (!p_) {
                 p_ = p;
-                size_ = bytes;
+                size_ = size;
                 dev_ = dev;
                 return;
             }
@@ -288,12 +291,13 @@ extern "C" int d4_xpattern_df(int n, const double *x, const double *y, const int
     const size_t vals = sizeof(double) * h.size(),
                  cells = sizeof(double2) * 2 * slices * (size_t)K * K;
     char *dev = nullptr;  // F, then the uploaded values
+    size_t size = 0;
     int st = D4_OK;
     auto ok = [&](cudaError_t e) {
         if (e != cudaSuccess && st == D4_OK) st = D4_ERR_CUDA;
         return e == cudaSuccess;
     };
-    if (ok(g_spare.take(&dev, cells + vals))) {
+    if (ok(g_spare.take(&dev, cells + vals, &size))) {
         double2 *F = reinterpret_cast<double2 *>(dev);
         double *dv = reinterpret_cast<double *>(dev + cells), *dacc = dv + 2 * (size_t)n;
         ok(cudaMemcpy(dv, h.data(), vals, cudaMemcpyHostToDevice));
@@ -306,6 +310,6 @@ extern "C" int d4_xpattern_df(int n, const double *x, const double *y, const int
             ok(cudaMemcpy(acc, dacc, sizeof(double) * 4 * K, cudaMemcpyDeviceToHost));
         }
     }
-    g_spare.give(dev, cells + vals, st == D4_OK);
+    g_spare.give(dev, size, st == D4_OK);
     return st;
 }
