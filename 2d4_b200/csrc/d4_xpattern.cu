@@ -12,6 +12,7 @@
 // shared memory (sincospi of 2 k v, so large k v keep their accuracy) and multiplies
 // on the FP64 matrix units; k_xp_sum adds the four |F|^2 over ky into the caller's
 // running sums.  No atomics, fixed orders: the result repeats bit for bit.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -200,60 +201,85 @@ __global__ void __launch_bounds__(128) k_xp_sum(int K, int slices, const double2
     }
 }
 
+// The driver's process-wide unique number of the allocation at p; 0 when there is none
+// or it cannot be queried.
+unsigned long long buffer_id(const void *p) {
+    using Fn = CUresult (*)(void *, CUpointer_attribute, CUdeviceptr);
+    static const Fn fn = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &f, cudaEnableDefault, &q) !=
+                cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            return (Fn) nullptr;
+        return reinterpret_cast<Fn>(f);
+    }();
+    unsigned long long id = 0;
+    if (!fn || fn(&id, CU_POINTER_ATTRIBUTE_BUFFER_ID, (CUdeviceptr)p) != CUDA_SUCCESS) return 0;
+    return id;
+}
+
 // The device block kept between calls: allocating and freeing one took 0.6 of the
 // 1.16 ms of a call (K = 513, n = 4096).  One block of at most kKeep bytes for the
 // whole process; a call has it to itself from take to give (a second thread's call
 // allocates its own), every call ends with its device work done, and another device,
-// a larger size, a failed allocation of the library or the process's end frees it.
+// a larger size or a failed allocation of the library frees it.  A device reset by the
+// host program frees it too, behind our back, and its address may become another
+// allocation's: the block is ours only while its buffer number is the one noted.
 class Spare {
   public:
     // *size: the block's own size, at least `bytes`; give gets it back.
     cudaError_t take(char **p, size_t bytes, size_t *size) {
         int dev = -1;
         cudaGetDevice(&dev);
-        {
-            std::lock_guard<std::mutex> lock(m_);
-            if (p_ && dev_ == dev && size_ >= bytes) {
-                *p = p_;
-                *size = size_;
-                p_ = nullptr;
-                return cudaSuccess;
-            }
+        Block b = grab();
+        if (b.p && b.dev == dev && b.size >= bytes) {
+            *p = b.p;
+            *size = b.size;
+            return cudaSuccess;
         }
-        release();
+        if (b.p) cudaFree(b.p);
         *size = bytes;
         return dmalloc(p, bytes);
     }
     void give(char *p, size_t size, bool keep) {
-        int dev = -1;
+        Block b{p, size, -1, 0};
         if (!p) return;
-        if (keep && size <= kKeep && cudaGetDevice(&dev) == cudaSuccess) {
+        if (keep && size <= kKeep && cudaGetDevice(&b.dev) == cudaSuccess &&
+            (b.id = buffer_id(p)) != 0) {
             std::lock_guard<std::mutex> lock(m_);
-            if (!p_) {
-                p_ = p;
-                size_ = size;
-                dev_ = dev;
+            if (!b_.p) {
+                b_ = b;
                 return;
             }
         }
         cudaFree(p);
     }
     void release() {
-        char *p = nullptr;
-        {
-            std::lock_guard<std::mutex> lock(m_);
-            std::swap(p, p_);
-        }
-        if (p) cudaFree(p);
+        const Block b = grab();
+        if (b.p) cudaFree(b.p);
     }
     ~Spare() { release(); }
 
   private:
+    struct Block {
+        char *p;
+        size_t size;
+        int dev;
+        unsigned long long id;
+    };
+    Block grab() {
+        Block b{};
+        {
+            std::lock_guard<std::mutex> lock(m_);
+            std::swap(b, b_);
+        }
+        if (b.p && buffer_id(b.p) != b.id) b = Block{};
+        return b;
+    }
     static constexpr size_t kKeep = 32u << 20;
     std::mutex m_;
-    char *p_ = nullptr;
-    size_t size_ = 0;
-    int dev_ = -1;
+    Block b_{};
 };
 Spare g_spare;
 
