@@ -223,8 +223,9 @@ unsigned long long buffer_id(const void *p) {
 // 1.16 ms of a call (K = 513, n = 4096).  One block of at most kKeep bytes for the
 // whole process; a call has it to itself from take to give (a second thread's call
 // allocates its own), every call ends with its device work done, and another device,
-// a larger size or a failed allocation of the library frees it.  A device reset by the
-// host program frees it too, behind our back, and its address may become another
+// a larger size or a failed allocation of the library frees it (the process's end does
+// by itself: the runtime must not be called after main).  A device reset by the host
+// program frees it too, behind our back, and its address may become another
 // allocation's: the block is ours only while its buffer number is the one noted.
 class Spare {
   public:
@@ -259,7 +260,6 @@ class Spare {
         const Block b = grab();
         if (b.p) cudaFree(b.p);
     }
-    ~Spare() { release(); }
 
   private:
     struct Block {
