@@ -109,13 +109,22 @@ void dalloc(T **p, size_t count) {
     D4_CUDA_OK(d4::dmalloc((void **)p, sizeof(T) * (count > 0 ? count : 1)));
 }
 
+// The factors of an FP64 LU and behind them its buffers, which it returns: Q (n x 64),
+// U12 (64 x n), the diagonal block, P0 (n x 32).  In one allocation, because creation
+// pays for each region of 2 MB that a further one opens (0.2 ms).
+double *dalloc_lu(double **lu, int n) {
+    const size_t nn = ((size_t)n * n + 15) / 16 * 16;
+    dalloc(lu, nn + (size_t)n * 160 + d4::kLuDiagWords);
+    return *lu + nn;
+}
+
 void free_all(Ctx *c) {
     void *bufs[] = {c->x0, c->y, c->xb, c->xh, c->x2, c->xs_tmp, c->ys_tmp, c->v_init,
                     c->v_init2, c->speed, c->speed2, c->dvec, c->dvec_new, c->fac, c->dx,
                     c->tol, c->A, c->LU, c->F, c->piv, c->perm, c->flags, c->red,
                     c->wave_err, c->xw1, c->xw2,
                     c->rowsub, c->rowsc,
-                    c->lu_q, c->lu_mask, c->lu_bar, c->A32, c->LU32, c->lu32_p0,
+                    c->lu_mask, c->lu_bar, c->A32, c->LU32, c->lu32_p0,
                     c->lu32_q, c->m_g, c->m_r, c->m_dx, c->m_c32, c->m_w1, c->m_resid,
                     c->m_part, c->m_dx2, c->m_cnt, c->m_conv, c->spiv};
     for (void *b : bufs)
@@ -125,7 +134,7 @@ void free_all(Ctx *c) {
     d4::blu_free(c->m32b.blu);
     if (c->blu_tasks) cudaFree(c->blu_tasks);
     const d4::Mix32Bufs &B = c->m32b;
-    void *ob[] = {c->lub.LU, c->lub.Q, c->lub.mask, c->lub.bar, c->lub.perm,
+    void *ob[] = {c->lub.LU, c->lub.mask, c->lub.bar, c->lub.perm,
                   c->lub.piv, c->flags3, c->F_b, c->dvec_b, c->speed_b, c->speed2_b, c->xw1_b,
                   c->xw2_b, c->dx_b, B.A32, B.LU32, B.P0, B.Q, B.mask, B.bar, B.perm, B.piv,
                   B.g, B.r, B.dx, B.part, B.c32, B.w1, B.resid, B.dx2, B.cnt, B.conv, B.A64,
@@ -827,7 +836,7 @@ int d4_create(void **out, int n, const d4_params *p) {
         // both forms: the FP64 matrix and pair-force scratch of the FP64 sweeps;
         // the FP64 factors only in the FP64 form
         dalloc(&c->A, nn);
-        dalloc(&c->LU, nn);  // the mixed form's FP64 attempts factorise here too
+        c->lu_q = dalloc_lu(&c->LU, n);  // the mixed form's FP64 attempts factorise here too
         dalloc(&c->F, nn);
         if (mixed) {
             dalloc(&c->A32, nn);
@@ -875,7 +884,6 @@ int d4_create(void **out, int n, const d4_params *p) {
         D4_CUDA_OK(cudaMemset(c->flags, 0, sizeof(int) * d4::kFlagCount));
         c->lu_grid = d4::coop_grid_size(n);
         if (c->lu_grid < 0) throw d4::StateError("n too large for the cooperative LU");
-        dalloc(&c->lu_q, (size_t)n * 160 + d4::kLuDiagWords);
         c->lu_p0 = c->lu_q + (size_t)n * 128 + d4::kLuDiagWords;
         d4::lu_encode_maps(c->lu_maps, c->LU, c->lu_q + (size_t)n * 64, n);
         c->lu_mask_words = d4::lu_mask_words_for(nblk);
@@ -912,8 +920,7 @@ int d4_create(void **out, int n, const d4_params *p) {
             if (!mixed || n < kMixedMinN) {
                 // the FP64 form's stage I (also the mixed form's attempts below
                 // kMixedMinN, which run on the FP64 path)
-                dalloc(&c->lub.LU, nn);
-                dalloc(&c->lub.Q, (size_t)n * 160 + d4::kLuDiagWords);
+                c->lub.Q = dalloc_lu(&c->lub.LU, n);
                 c->lub.P0 = c->lub.Q + (size_t)n * 128 + d4::kLuDiagWords;
                 dalloc(&c->lub.mask, (size_t)c->lu_mask_words);
                 dalloc(&c->lub.bar, 64);
