@@ -161,15 +161,19 @@ __device__ __forceinline__ double xy_diff_x(double dx, double dy, const Hyp &h, 
 // ---- the pair tiles' evaluation ----
 //
 // pair() gives xy and, with kGrad, xy_diff_x of one pair: the same expressions in
-// the same order as above, every quotient the correctly rounded one, from one
-// reciprocal per image instead of a division each (44 divisions a pair for both
-// values, with a slow-path branch each; the fused tiles ran 1,680 instructions a
-// pair at 152 registers, one block per SM, 30% of the issue slots).  A quotient
-// is q0 = a y, q = q0 + (a - b q0) y with the residual exact in one FMA: with y
-// within 2^-51 of 1/b, q is RN(a/b) unless a/b lies within 2^-49 ulp of the
-// middle of two doubles.
+// the same order as above, with one reciprocal per image instead of a division per
+// quotient (44 divisions a pair for both values, with a slow-path branch each; the
+// fused tiles ran 1,680 instructions a pair at 152 registers, one block per SM, 30% of
+// the issue slots).  A quotient is q0 = a y, q = q0 + (a - b q0) y (Markstein 1990).
+// With u = 2^-53, y is within u of 1/b for b = q, 4 u for b = q^2 (y y) and 7 u for
+// b = q^3 (y y y), relative.  So q0 is within 2, 5 and 8 of the distances of two
+// doubles from a/b, the last step brings that to 2^-51, 2^-48 and 2^-47 before its
+// rounding, and q is the correctly rounded quotient except where a/b lies nearer than
+// that to the middle of two doubles: there it may be the other neighbour (about one
+// quotient in 10^14).
 
-// 1/b within an ulp: Newton steps from the hardware's estimate.
+// 1/b: Newton steps from the hardware's estimate (relative error 2^-20, then 2^-40 and
+// below 2^-79, and the rounding of the last step).
 __device__ __forceinline__ double recip(double b) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));

@@ -50,7 +50,8 @@ __device__ __forceinline__ D dsinh(D x) { return D{sinh(x.v), cosh(x.v) * x.d}; 
 using f64::kPi;
 
 // Quotients of the images (divisors far inside the normal range): both parts from
-// one reciprocal, correctly rounded as a division's (d4_field64.cuh).
+// one reciprocal, correctly rounded but beside the middle of two doubles
+// (d4_field64.cuh).
 __device__ __forceinline__ D ratio(D a, D b) {
     const double y = f64::recip(b.v);
     const double q = f64::quot(a.v, b.v, y);
