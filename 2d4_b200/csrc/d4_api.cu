@@ -230,7 +230,8 @@ constexpr int kMixedMinN = 2048;
 // Grid split of an attempt's two concurrent cooperative factorisations:
 // stage I's chain (one LU, two solves, one sweep) is the shorter one, so it
 // gets 40% of the co-resident CTAs and stage II's factorisation the rest.
-// Neither gets fewer than one thread per row (n / 256 CTAs).
+// Neither gets fewer than one thread per row (n / 256 CTAs), as the pivoted FP32 LU
+// needs.
 static void stage_split(int grid, int n, int &g1, int &g2) {
     const int need = (n + 255) / 256;
     g1 = std::max(need, grid * 2 / 5);
@@ -882,8 +883,8 @@ int d4_create(void **out, int n, const d4_params *p) {
         D4_CUDA_OK(cudaMemset(c->F, 0, sizeof(double) * nn));
         D4_CUDA_OK(cudaMemset(c->dvec, 0, sizeof(double) * n));
         D4_CUDA_OK(cudaMemset(c->flags, 0, sizeof(int) * d4::kFlagCount));
-        c->lu_grid = d4::coop_grid_size(n);
-        if (c->lu_grid < 0) throw d4::StateError("n too large for the cooperative LU");
+        c->lu_grid = d4::coop_grid_size();
+        if (c->lu_grid < 0) throw d4::StateError("no CTA of the cooperative LU fits an SM");
         c->lu_p0 = c->lu_q + (size_t)n * 128 + d4::kLuDiagWords;
         d4::lu_encode_maps(c->lu_maps, c->LU, c->lu_q + (size_t)n * 64, n);
         c->lu_mask_words = d4::lu_mask_words_for(nblk);

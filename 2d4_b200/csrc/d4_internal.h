@@ -317,7 +317,7 @@ inline void count_lu(Ctx &c, const int *fl) {
     c.lu_passes += fl[kFlagPasses];
     c.lu_swaps += fl[kFlagSwaps];
 }
-int coop_grid_size(int n);            // CTAs of the cooperative LU (-1: n too large)
+int coop_grid_size();  // CTAs of the FP64 cooperative LU (-1: none fits)
 enum GMode { kGBig = 0, kGHalf = 1, kGNewton = 2 };
 // g built from (gmode, hval, dvec, s_end, s_init, x_new, x_old); solve; out = base - dx.
 void solve_update64(Ctx &c, int gmode, double hval, const double *s_end, const double *s_init,

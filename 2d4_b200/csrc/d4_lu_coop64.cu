@@ -73,7 +73,7 @@ void lu_encode_maps(LuMaps &m, double *A, double *U, int n) {
     one(m.u, U, 2 * lux::NB, lux::kBoxC, lux::NB);
 }
 
-int coop_grid_size(int n) {
+int coop_grid_size() {
     int dev = 0, sms = 0, per_sm = 0;
     D4_CUDA_OK(cudaGetDevice(&dev));
     D4_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

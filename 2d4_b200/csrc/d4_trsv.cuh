@@ -30,16 +30,6 @@ __device__ __forceinline__ double g_of(const GArgs &ga, int r) {
     return ga.x_new[r] - ga.x_old[r] - ga.hval * X / 2;
 }
 
-__device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ void st_release(unsigned *p, unsigned v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
 constexpr long long kSpinLimit = 1ll << 25;  // polls: > 1 s
 
 // ---------------------------------------------------------------------------

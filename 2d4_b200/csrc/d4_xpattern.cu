@@ -29,7 +29,6 @@ constexpr int kXpThin = 16;   // thin tiles along a short remainder of K: kXpThi
 constexpr int kXpLong = 128;
 constexpr int kXpChunk = 32;  // dislocations staged per step
 constexpr int kXpThreads = 512;
-constexpr int kXpBlocks = 148;  // blocks aimed at when the tiles are few: one per SM
 // the factors of a tile's rows and columns for one dislocation; 2 mod 8: no bank
 // conflicts
 __host__ __device__ constexpr int xp_row(int m, int n) { return m + n + 2; }
@@ -310,10 +309,14 @@ extern "C" int d4_xpattern_df(int n, const double *x, const double *y, const int
     }
     std::copy(acc, acc + 4 * (size_t)K, h.begin() + 2 * (size_t)n);
     const int tiles = XpTiles(K).count();
+    int dev_no = 0, sms = 0;
+    if (cudaGetDevice(&dev_no) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_no) != cudaSuccess)
+        return D4_ERR_CUDA;
     // few tiles: the dislocations are cut into slices, so that about one block runs
     // per SM, of at least four chunks each (below that the sums over the slices and
     // the first chunk's latency weigh as much as the products)
-    const int slices = std::max(1, std::min(kXpBlocks / (2 * tiles), n / (4 * kXpChunk)));
+    const int slices = std::max(1, std::min(sms / (2 * tiles), n / (4 * kXpChunk)));
     const size_t vals = sizeof(double) * h.size(),
                  cells = sizeof(double2) * 2 * slices * (size_t)K * K;
     char *dev = nullptr;  // F, then the uploaded values
