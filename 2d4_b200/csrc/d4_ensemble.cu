@@ -224,8 +224,8 @@ __global__ void __launch_bounds__(lux::kThreads, 1) k_ens_lu(Pools P, const Inst
     a.flags = P.lu_flags + k * kFlagCount;
     a.map_a = &P.lu_maps[k].a;
     a.map_u = &P.lu_maps[k].u;
-    if (threadIdx.x == 0) {
-        // tensor maps in global memory: acquired by the thread that uses them
+    if (threadIdx.x % 32 == 0) {
+        // tensor maps in global memory: acquired by the threads that issue the copies
         asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(a.map_a)
                      : "memory");
         asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(a.map_u)
