@@ -12,7 +12,7 @@
 // Schedule, per block of 32 columns:
 //   pass    Without pivoting, from the diagonal block's factors: the rows below
 //           it (multipliers L21) and the columns right of it (U12 = L11^-1 A12),
-//           8 lanes per row or column, both by all warps at once.  Starts from
+//           4 lanes per row or column, both by all warps at once.  Starts from
 //           a saved copy P0 of the block's columns with the swaps found so far
 //           applied; U12 goes to a buffer, so a rejected pass has overwritten
 //           nothing it reads.  Pre-division values go to Q; a 32-bit mask
@@ -31,7 +31,8 @@
 //           (the same operations in the same order as the tile that owns it),
 //           eliminates it and publishes it.  The oracle skips an update whose
 //           u_kj is exactly 0; here it is applied (x - l*0 == x for finite l,
-//           and the multipliers of an accepted pass are finite: |l| <= 1).
+//           and the multipliers of an accepted pass are finite, |l| <= 1, while the
+//           elimination stays finite; the slow paths of a pass do skip).
 // The next block's pass waits for that publication and those tiles only, so a
 // block without swaps costs one group barrier.  Every wait is bounded.
 //
@@ -322,7 +323,7 @@ __device__ __forceinline__ uint32_t mbar_wait(uint64_t *b, uint32_t parity) {
 // next pivot's product and difference: every lane forms the next pivot itself
 // from values broadcast a step early, and its reciprocal's seed starts from the
 // uncorrected quotient, so no shuffle and no seed latency stays in the chain
-// (240 cycles per column measured for the whole block, 406 with an IEEE
+// (275 cycles per column measured for the whole block, 406 with an IEEE
 // division, a shuffle and a CTA barrier per column).  Pads (rows and columns
 // >= kw) are those of an identity.  Returns the thread's flags: columns where a
 // row has |a_ik| > |a_kk|, which for correctly rounded quotients is |l| > 1.

@@ -13,7 +13,7 @@
 // Every solve of the step then runs GMRES(40) with right Jacobi preconditioning,
 // classical Gram-Schmidt with one reorthogonalisation and Givens rotations, to a
 // relative residual of 1e-13, as one cooperative kernel: each CTA owns a
-// contiguous range of rows, the SpMV is one warp per row (fixed lane split and
+// contiguous range of rows, the SpMV is 8 lanes per row (fixed lane split and
 // butterfly, so results do not depend on timing), and each reduction goes
 // through per-CTA partials (double-buffered) and a bounded grid barrier, three
 // barriers per Krylov vector.  A solve that does not converge within the restart
@@ -101,8 +101,9 @@ __device__ __forceinline__ void spmv_rows(const GmresArgs &a, int r0, int rows, 
     __syncthreads();
 }
 
-// Bound by the three grid barriers of a Krylov vector (1.3 us each over 128 CTAs)
-// and the reductions around them.  32 rows per CTA, so that one pass of the SpMV
+// Bound by the chain of a Krylov vector, 17 us at N = 4096: three reductions over 128
+// CTAs, whose barriers take 1.3 us each, with the sums on both sides of them, and the
+// SpMV's gathers.  32 rows per CTA, so that one pass of the SpMV
 // covers them with 8 lanes a row, the basis in shared memory (rows of a CTA only), a
 // warp per dot product and per total: N = 4096 486 -> 236 us a solve (128 rows per
 // CTA with one warp per row, the basis in memory, every total a serial sum, and a

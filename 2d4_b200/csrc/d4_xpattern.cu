@@ -5,13 +5,14 @@
 // With K = res/2 + 1 and the four densities m = rho_t (weight 1), kappa
 // (weight b), rho_p (b = +1 only) and rho_n (b = -1 only),
 //     F_m(kx, ky) = sum_i w_m(b_i) exp(-2 pi i (kx x_i + ky y_i)),
-//     S_m(kx)    += sum_ky |F_m(kx, ky)|^2     (over ky ascending).
+//     S_m(kx)    += sum_ky |F_m(kx, ky)|^2.
 // F_p and F_n (the sums over the b = +1 and the other dislocations; rho_t = F_p +
 // F_n, kappa = F_p - F_n) are complex matrix products Ex^T Ey over their
 // dislocations with E[i][k] = exp(-2 pi i k v_i).  k_xp_gemm forms both factors in
 // shared memory (sincospi of 2 k v, so large k v keep their accuracy) and multiplies
-// on the FP64 matrix units; k_xp_sum adds the four |F|^2 over ky into the caller's
-// running sums.  No atomics, fixed orders: the result repeats bit for bit.
+// on the FP64 matrix units; k_xp_sum adds the four |F|^2 over ky (every 32nd per lane,
+// then a tree) into the caller's running sums.  No atomics, fixed orders: the result
+// repeats bit for bit.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
