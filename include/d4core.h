@@ -314,12 +314,13 @@ int d4_ensemble_run(void *ens, long long max_rounds, d4_run_result *res);
  * xpattern tool, method df, xpattern/xpattern.cpp:393-423).  With K = res/2+1
  * and F_m(kx, ky) = sum_i w_m(b_i) exp(-2 pi i (kx x_i + ky y_i)) for the four
  * densities m = rho_t (w = 1), kappa (w = b), rho_p (b = +1) and rho_n
- * (b = -1), adds sum_ky |F_m(kx, ky)|^2 (ky ascending) to acc[m*K + kx],
+ * (b = -1), adds sum_ky |F_m(kx, ky)|^2 (in a fixed order) to acc[m*K + kx],
  * kx = 0..K-1, so that repeated calls sum over configurations as the tool
  * does over its input files.  x, y, b: host arrays of n entries; acc: host,
  * 4*K entries, read and updated.  FP64 throughout; 2 <= res <= 65536.  Uses
- * the current device and allocates its scratch (two n x K tables and 4 K^2
- * doubles) for the call. */
+ * the current device; its scratch (4 K^2 doubles, more for few wave numbers, and
+ * the inputs) is allocated for the call, or is the block of at most 32 MB that the
+ * library keeps from an earlier one. */
 int d4_xpattern_df(int n, const double *x, const double *y, const int *b, int res, double *acc);
 
 /* Schedule of an attempt (dense plain and mixed forms): enable = 1 (the
